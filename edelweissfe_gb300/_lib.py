@@ -36,6 +36,7 @@ EXPORTS = [
     "efe_accept_state",
     "efe_fma_probe",
     "efe_csr_spmv",
+    "efe_pcg_solve",
     "efe_pcg_start",
     "efe_pcg_iterate",
     "efe_csr_gemv",
@@ -204,6 +205,8 @@ def load(build_if_missing=False):
     lib.efe_pcg_start.argtypes = [ctypes.POINTER(EfePcg), P, P]
     lib.efe_pcg_iterate.restype = i32
     lib.efe_pcg_iterate.argtypes = [ctypes.POINTER(EfePcg), i64, i32, P]
+    lib.efe_pcg_solve.restype = i32
+    lib.efe_pcg_solve.argtypes = [ctypes.POINTER(EfePcg), P, i64, i64, i32, i32, f64, P]
     lib.efe_csr_gemv.restype = i32
     lib.efe_csr_gemv.argtypes = [ctypes.POINTER(EfeCsr), P, f64, f64, P, P]
     lib.efe_csr_gemv_pairs.restype = i32

@@ -596,8 +596,20 @@ int32_t efe_pcg_iterate(const EfePcg* s, int64_t firstIteration, int32_t nIterat
   if (rc) return rc;
   if (firstIteration < 0 || nIterations < 0) return fail(EFE_ERR_ARGUMENT, "negative iteration count");
   if (s->n == 0) return EFE_OK;
-  cudaError_t e = efe::pcg_iterate(*s, firstIteration, nIterations, (cudaStream_t)stream);
+  cudaError_t e = efe::pcg_run(*s, nullptr, 0, firstIteration, nIterations, 0, 0.0, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "efe_pcg_iterate");
+  return EFE_OK;
+}
+
+int32_t efe_pcg_solve(const EfePcg* s, const int32_t* blockCols, int64_t nnz, int64_t firstIteration,
+                      int32_t nIterations, int32_t every, double tol2, void* stream) {
+  int32_t rc = check_pcg(s);
+  if (rc) return rc;
+  if (firstIteration < 0 || nIterations < 0 || nnz < 0) return fail(EFE_ERR_ARGUMENT, "negative iteration or entry count");
+  if (every < 1) return fail(EFE_ERR_ARGUMENT, "every must be at least 1");
+  if (s->n == 0) return EFE_OK;
+  cudaError_t e = efe::pcg_run(*s, blockCols, nnz, firstIteration, nIterations, every, tol2, (cudaStream_t)stream);
+  if (e != cudaSuccess) return cuda_fail(e, "efe_pcg_solve");
   return EFE_OK;
 }
 

@@ -279,6 +279,25 @@ __device__ __forceinline__ ff ff_split_bits(double x) {
   return ff_split(x);
 }
 
+// double -> (hi, lo) with hi = fl32(x) rounded to nearest (ties away from zero) and lo = fl32(x - hi):
+// ff_split's accuracy (~2^-49 relative) with integer and FP32 instructions.  x - hi is the low 29
+// fraction bits, less 2^29 where hi was rounded up, times 2^(E - 1075).
+__device__ __forceinline__ ff ff_split_rn_bits(double x) {
+  const uint64_t X = (uint64_t)__double_as_longlong(x);
+  const uint32_t E = (uint32_t)(X >> 52) & 0x7ffu;
+  if (E - 949u < 201u) {
+    const uint64_t mag = X & 0x7fffffffffffffffull;
+    const uint32_t sign = (uint32_t)(X >> 32) & 0x80000000u;
+    const float h = __uint_as_float(sign | ((uint32_t)((mag + (1ull << 28)) >> 29) - (896u << 23)));
+    int32_t rem = (int32_t)((uint32_t)mag & 0x1fffffffu);
+    if (rem >= 1 << 28) rem -= 1 << 29;
+    const float l = __fmul_rn(__int2float_rn(sign ? -rem : rem), __uint_as_float((E - 948u) << 23));
+    return ff{h, l};
+  }
+  if ((X << 1) == 0ull) return ff{__uint_as_float((uint32_t)(X >> 32)), 0.0f};
+  return ff_split(x);
+}
+
 // hi + lo as a double: exact conversions, one rounding add
 __device__ __forceinline__ double ff_to_double_bits(ff a) { return f2d_bits(a.h) + f2d_bits(a.l); }
 

@@ -242,7 +242,10 @@ cudaError_t chebyshev_step(int64_t n, const double* dinv, const double* r, doubl
                            double* d, double* z, float2* dff, cudaStream_t st);
 cudaError_t split_pairs(int64_t n, const double* x, float2* xf, cudaStream_t st);
 cudaError_t pcg_start(const EfePcg& s, const double* b, cudaStream_t st);
-cudaError_t pcg_iterate(const EfePcg& s, int64_t k0, int nIter, cudaStream_t st);
+// CG iterations (efe_pcg.cu); blockCols: first column of every node block or null; every > 0: test
+// r.r <= tol2 each `every` iterations and stop one such batch later
+cudaError_t pcg_run(const EfePcg& s, const int32_t* blockCols, int64_t nnz, int64_t k0, int nIter, int every, double tol2,
+                    cudaStream_t st);
 cudaError_t adjoint_ss_quad4(int rule, const SSAdjointArgs& a, cudaStream_t st);
 cudaError_t adjoint_ss_quad8(int rule, const SSAdjointArgs& a, cudaStream_t st);
 cudaError_t adjoint_ss_hexa8(int rule, const SSAdjointArgs& a, cudaStream_t st);

@@ -25,11 +25,8 @@
 // y = alpha A x + beta y (rectangular for the transfer operators, masked for the tangent) and the
 // vector step of a Chebyshev smoother; the host composes them into V-cycles.
 //
-// One iteration is three kernels: (1) Ap = A p with the partial sums of p.Ap per block, (2) alpha,
-// x += alpha p, r -= alpha Ap, z = M^-1 r with the partial sums of r.z and r.r, (3) beta,
-// p = z + beta p.  The scalars stay on the device: every block sums the previous kernel's partials
-// in the same fixed order, so the iteration is deterministic, and rz is double-buffered by the
-// parity of the iteration number so no kernel overwrites a scalar another block is reading.
+// The iterations themselves are one persistent kernel (efe_pcg.cu); here are their start, the products
+// and the smoother step.
 #include "efe_launch.cuh"
 
 namespace efe {
@@ -39,8 +36,8 @@ namespace {
 constexpr int NT = 256;                 // threads per block of every kernel here
 constexpr int WARPS = NT / 32;
 constexpr int MAX_BLOCKS = 2048;        // partial-sum slots per reduction
-// work layout (doubles): [0..1] rz (by parity), [2] r.r, [3] p.Ap, [8 ..) three partial arrays
-constexpr int PART0 = 8, PART1 = PART0 + MAX_BLOCKS, PART2 = PART1 + MAX_BLOCKS;
+// work layout: efe_pcg.cu
+constexpr int PART1 = 8 + MAX_BLOCKS, PART2 = PART1 + MAX_BLOCKS;
 
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -186,76 +183,23 @@ __device__ __forceinline__ void group_product_ff(const int32_t* __restrict__ ind
   }
 }
 
-// The float-float CG product over node row groups of PB rows (spmv_kernel<float, true> otherwise).
-template <int PB>
-__global__ void __launch_bounds__(NT) spmv_group_ff_kernel(int64_t n, const int32_t* __restrict__ indptr,
-                                                           const int32_t* __restrict__ indices,
-                                                           const float* __restrict__ K,
-                                                           const uint8_t* __restrict__ freeMask,
-                                                           const double* __restrict__ x, const float2* __restrict__ xf,
-                                                           double* __restrict__ y, double* part) {
-  __shared__ double sh[WARPS + 1];
-  const int lane = threadIdx.x % 32, g = lane / G, sl = lane % G;
-  constexpr int GPW = 32 / G;  // row groups per warp and step
-  const int64_t warp = ((int64_t)blockIdx.x * NT + threadIdx.x) / 32;
-  const int64_t nw = (int64_t)gridDim.x * WARPS;
-  const int64_t nGroups = n / PB;
-  double acc = 0.0;
-  // the loop condition depends on the warp only: all 32 lanes reach every shuffle
-  for (int64_t gb = warp * GPW; gb < nGroups; gb += nw * GPW) {
-    const int64_t gi = gb + g;
-    const bool live = gi < nGroups;
-    double v[PB];
-    group_product_ff<PB>(indptr, gi * PB, live, indices, K, xf, sl, v);
-    if (live && sl == 0) {
-#pragma unroll
-      for (int c = 0; c < PB; ++c) {
-        const int64_t r = gi * PB + c;
-        const double yr = (!freeMask || freeMask[r]) ? v[c] : x[r];
-        y[r] = yr;
-        acc = fma(x[r], yr, acc);
-      }
-    }
-  }
-  if (part) {
-    const double s = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-  }
-}
-
-// y_r = free_r ? (K x)_r : x_r for rows r; with part != null also the block partials of x.y.
-// FF: x is also given as the float-float pairs xf and K is float (the CG iterations of FP32 tangents).
-template <typename KT, bool FF>
+// y_r = free_r ? (K x)_r : x_r for rows r
+template <typename KT>
 __global__ void __launch_bounds__(NT) spmv_kernel(int64_t n, const int32_t* __restrict__ indptr,
                                                   const int32_t* __restrict__ indices, const KT* __restrict__ K,
                                                   const uint8_t* __restrict__ freeMask, const double* __restrict__ x,
-                                                  const float2* __restrict__ xf, double* __restrict__ y,
-                                                  double* part) {
-  __shared__ double sh[WARPS + 1];
+                                                  double* __restrict__ y) {
   const int lane = threadIdx.x % 32, g = lane / G, sl = lane % G;
   constexpr int RPW = 32 / G;  // rows per warp and step
   const int64_t warp = ((int64_t)blockIdx.x * NT + threadIdx.x) / 32;
   const int64_t nw = (int64_t)gridDim.x * WARPS;
-  double acc = 0.0;
   // the loop condition depends on the warp only: all 32 lanes reach every shuffle
   for (int64_t rb = warp * RPW; rb < n; rb += nw * RPW) {
     const int64_t r = rb + g;
     const bool live = r < n;
     const int32_t b = live ? indptr[r] : 0, e = live ? indptr[r + 1] : 0;
-    double v;
-    if constexpr (FF)
-      v = row_product_ff(b, e, indices, reinterpret_cast<const float*>(K), xf, sl);
-    else
-      v = row_product(b, e, indices, K, x, sl);
-    if (live && sl == 0) {
-      const double yr = (!freeMask || freeMask[r]) ? v : x[r];
-      y[r] = yr;
-      acc = fma(x[r], yr, acc);
-    }
-  }
-  if (part) {
-    const double s = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    const double v = row_product(b, e, indices, K, x, sl);
+    if (live && sl == 0) y[r] = (!freeMask || freeMask[r]) ? v : x[r];
   }
 }
 
@@ -320,69 +264,7 @@ __global__ void __launch_bounds__(NT) pcg_start_finish(double* work, int nb) {
     work[0] = rz;
     work[1] = 0.0;
     work[2] = rr;
-    work[3] = 0.0;
-  }
-}
-
-// alpha = rz[cur] / p.Ap; x += alpha p; r -= alpha Ap; z = M^-1 r; partials of r.z (PART1), r.r (PART2)
-template <int BS>
-__global__ void __launch_bounds__(NT) pcg_update_kernel(int64_t n, int cur, int nbSpmv, const double* __restrict__ p,
-                                                        const double* __restrict__ Ap, const double* __restrict__ dinv,
-                                                        double* __restrict__ x, double* __restrict__ r,
-                                                        double* __restrict__ z, double* work) {
-  __shared__ double sh[WARPS + 1];
-  const double pAp = sum_partials(work + PART0, nbSpmv, sh);
-  const double alpha = pAp != 0.0 ? work[cur] / pAp : 0.0;
-  double rz = 0.0, rr = 0.0;
-  const int64_t nb = n / BS;
-  for (int64_t k = (int64_t)blockIdx.x * NT + threadIdx.x; k < nb; k += (int64_t)gridDim.x * NT) {
-    double rv[BS], zv[BS];
-#pragma unroll
-    for (int c = 0; c < BS; ++c) {
-      const int64_t i = k * BS + c;
-      x[i] = fma(alpha, p[i], x[i]);
-      rv[c] = fma(-alpha, Ap[i], r[i]);
-      r[i] = rv[c];
-    }
-    precondition<BS>(dinv, k, rv, zv);
-#pragma unroll
-    for (int c = 0; c < BS; ++c) {
-      z[k * BS + c] = zv[c];
-      rz = fma(rv[c], zv[c], rz);
-      rr = fma(rv[c], rv[c], rr);
-    }
-  }
-  const double s1 = block_sum(rz, sh);
-  if (threadIdx.x == 0) work[PART1 + blockIdx.x] = s1;
-  const double s2 = block_sum(rr, sh);
-  if (threadIdx.x == 0) {
-    work[PART2 + blockIdx.x] = s2;
-    if (blockIdx.x == 0) work[3] = pAp;
-  }
-}
-
-// beta = rz_new / rz[cur]; p = z + beta p; block 0 stores rz_new in rz[cur ^ 1] and r.r in work[2]
-__global__ void __launch_bounds__(NT) pcg_direction_kernel(int64_t n, int cur, int nbVec, const double* __restrict__ z,
-                                                           double* __restrict__ p, float2* __restrict__ pf,
-                                                           double* work) {
-  __shared__ double sh[WARPS + 1];
-  const double rzNew = sum_partials(work + PART1, nbVec, sh);
-  const double rzOld = work[cur];
-  const double beta = rzOld != 0.0 ? rzNew / rzOld : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    const double pi = fma(beta, p[i], z[i]);
-    p[i] = pi;
-    if (pf) {  // float-float copy for the FP32 product: pi = h + l to ~48 bits
-      const float h = __double2float_rn(pi);
-      pf[i] = make_float2(h, __double2float_rn(pi - (double)h));
-    }
-  }
-  if (blockIdx.x == 0) {
-    const double rr = sum_partials(work + PART2, nbVec, sh);
-    if (threadIdx.x == 0) {
-      work[cur ^ 1] = rzNew;
-      work[2] = rr;
-    }
+    for (int k = 3; k < 8; ++k) work[k] = 0.0;  // no product yet, not ended, no iterations (efe_pcg.cu)
   }
 }
 
@@ -536,35 +418,7 @@ int sm_count() {
   return sms;
 }
 
-bool use_ff(const EfePcg& s) { return s.kPrecision != EFE_K_FP64 && s.pFF; }
-float2* pff(const EfePcg& s) { return use_ff(s) ? reinterpret_cast<float2*>(s.pFF) : nullptr; }
-
-template <typename KT, bool FF>
-cudaError_t spmv_t(const EfePcg& s, const double* x, const float2* xf, double* y, double* part, int nb,
-                   cudaStream_t st) {
-  spmv_kernel<KT, FF><<<nb, NT, 0, st>>>(s.n, s.indptr, s.indices, static_cast<const KT*>(s.Kdata), s.freeMask, x, xf,
-                                          y, part);
-  return cudaGetLastError();
-}
-
-// float-float product of an FP32 tangent, over node row groups where the pattern has them
-cudaError_t spmv_pairs(const EfePcg& s, const double* x, const float2* xf, double* y, double* part, int nb,
-                       cudaStream_t st) {
-  const float* K = static_cast<const float*>(s.Kdata);
-  if (s.patternBlock == 3 && s.n % 3 == 0)
-    spmv_group_ff_kernel<3><<<nb, NT, 0, st>>>(s.n, s.indptr, s.indices, K, s.freeMask, x, xf, y, part);
-  else if (s.patternBlock == 2 && s.n % 2 == 0)
-    spmv_group_ff_kernel<2><<<nb, NT, 0, st>>>(s.n, s.indptr, s.indices, K, s.freeMask, x, xf, y, part);
-  else
-    return spmv_t<float, true>(s, x, xf, y, part, nb, st);
-  return cudaGetLastError();
-}
-
-// FP64 arithmetic product (any x)
-cudaError_t spmv(const EfePcg& s, const double* x, double* y, double* part, int nb, cudaStream_t st) {
-  return s.kPrecision == EFE_K_FP64 ? spmv_t<double, false>(s, x, nullptr, y, part, nb, st)
-                                    : spmv_t<float, false>(s, x, nullptr, y, part, nb, st);
-}
+float2* pff(const EfePcg& s) { return s.kPrecision != EFE_K_FP64 && s.pFF ? reinterpret_cast<float2*>(s.pFF) : nullptr; }
 
 }  // namespace
 
@@ -619,7 +473,12 @@ cudaError_t split_pairs(int64_t n, const double* x, float2* xf, cudaStream_t st)
 
 cudaError_t csr_spmv(const EfePcg& s, const double* x, double* y, cudaStream_t st) {
   if (s.n == 0) return cudaSuccess;
-  return spmv(s, x, y, nullptr, spmv_blocks(s.n, sm_count()), st);
+  const int nb = spmv_blocks(s.n, sm_count());
+  if (s.kPrecision == EFE_K_FP64)
+    spmv_kernel<double><<<nb, NT, 0, st>>>(s.n, s.indptr, s.indices, static_cast<const double*>(s.Kdata), s.freeMask, x, y);
+  else
+    spmv_kernel<float><<<nb, NT, 0, st>>>(s.n, s.indptr, s.indices, static_cast<const float*>(s.Kdata), s.freeMask, x, y);
+  return cudaGetLastError();
 }
 
 cudaError_t pcg_start(const EfePcg& s, const double* b, cudaStream_t st) {
@@ -633,27 +492,6 @@ cudaError_t pcg_start(const EfePcg& s, const double* b, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   pcg_start_finish<<<1, NT, 0, st>>>(s.work, nb);
   return cudaGetLastError();
-}
-
-cudaError_t pcg_iterate(const EfePcg& s, int64_t k0, int nIter, cudaStream_t st) {
-  const int sms = sm_count();
-  const int nbS = spmv_blocks(s.n, sms), nbV = vec_blocks(s.n, sms);
-  float2* pf = pff(s);
-  for (int k = 0; k < nIter; ++k) {
-    const int cur = (int)((k0 + k) & 1);
-    cudaError_t e = pf ? spmv_pairs(s, s.p, pf, s.Ap, s.work + PART0, nbS, st)
-                       : spmv(s, s.p, s.Ap, s.work + PART0, nbS, st);
-    if (e != cudaSuccess) return e;
-    switch (s.blockSize) {
-      case 1: pcg_update_kernel<1><<<nbV, NT, 0, st>>>(s.n, cur, nbS, s.p, s.Ap, s.dinv, s.x, s.r, s.z, s.work); break;
-      case 2: pcg_update_kernel<2><<<nbV, NT, 0, st>>>(s.n, cur, nbS, s.p, s.Ap, s.dinv, s.x, s.r, s.z, s.work); break;
-      default: pcg_update_kernel<3><<<nbV, NT, 0, st>>>(s.n, cur, nbS, s.p, s.Ap, s.dinv, s.x, s.r, s.z, s.work); break;
-    }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    pcg_direction_kernel<<<nbV, NT, 0, st>>>(s.n, cur, nbV, s.z, s.p, pf, s.work);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
 }
 
 }  // namespace efe

@@ -166,9 +166,19 @@ class NISTGPU:
         # displacement components) -- on near-regular hexahedral meshes of isotropic material the
         # same-node couplings nearly cancel and both need the same iterations
         self.pcgPreconditioner = pcgPreconditioner
-        # replay the PCG iteration batches of long solves as one CUDA graph (same kernels and
+        # replay the iteration batches of multigrid CG solves as one CUDA graph (same kernels and
         # arguments as the direct launches, so the same results bit for bit)
         self.pcgGraphs = pcgGraphs
+        # first column of every node block of the pattern, where the rows and columns come in aligned
+        # blocks of a node's DOFs (efe_pcg_solve reads it instead of one index per entry)
+        self._block_cols = None
+        if getattr(assembler, "rowGroup", 1) > 1 and assembler.device.type == "cuda":
+            bs = assembler.rowGroup
+            start = assembler.indptr[::bs].to(torch.int64)  # first entry of every row group
+            count = (start[1:] - start[:-1]) // (bs * bs)
+            group = torch.repeat_interleave(torch.arange(len(count), device=assembler.device), count)
+            t = torch.arange(len(group), device=assembler.device) - (start[:-1] // (bs * bs))[group]
+            self._block_cols = assembler.indices[start[:-1][group] + bs * t].contiguous()
         # "amg": aggregation multigrid V-cycles (amg.AggregationAMG, built once per set of
         # prescribed DOFs, its level operators once per tangent)
         self.amgOptions = dict(amgOptions or {})
@@ -338,13 +348,10 @@ class NISTGPU:
         side gives the same solution from the symmetric positive-definite system on the free DOFs:
         x = x_d + y with x_d = R on the prescribed DOFs and K_ff y_f = R_f - K_fd x_d.  K is used as
         assembled (FP32 or FP64 values).  Converged when |r| <= pcgTolerance |b| (checked every
-        10 iterations, as b's norm includes the prescribed values).  The check of a batch is read
-        while the next batch already runs (its r.r copied to pinned memory behind the batch), so the
-        device never waits for the host; a converged solve therefore runs one batch past the batch
-        that met the tolerance (the kernels stop moving x when p.Ap or r.z reach zero).  With pcgGraphs, a solve still
-        running after its first 20 iterations captures one batch of 10 iterations (30 launches) as a
-        CUDA graph and replays it: the kernels read the iteration number only for its parity, which
-        is even at the start of every batch."""
+        10 iterations, as b's norm includes the prescribed values).  The test runs on the device
+        (efe_pcg_solve); a converged solve runs one batch of 10 iterations past the one that met the
+        tolerance.  One launch holds many iterations, and the host looks at the previous launch's
+        outcome while the next one already runs."""
         import ctypes
 
         from . import _lib as L
@@ -389,30 +396,31 @@ class NISTGPU:
         L.check(lib.efe_pcg_start(ctypes.byref(s), ctypes.c_void_p(b.data_ptr()), stream), "efe_pcg_start")
         tol2 = (self.pcgTolerance * bnorm) ** 2
         k = 0
-        graph = None
         if bnorm > 0.0 and float(work[2]) > tol2:
-            seen = torch.empty((2, 2), dtype=torch.float64, pin_memory=True)  # r.r, p.Ap of two batches
+            cols = ctypes.c_void_p(self._block_cols.data_ptr() if self._block_cols is not None else None)
+            # one launch runs about 20 ms of iterations (and returns early once the solve has ended)
+            seconds = 4e-6 + asm.nnz * K.element_size() / 4e12
+            segment = 10 * min(200, max(5, int(2e-3 / seconds)))
+            seen = torch.empty((2, 6), dtype=torch.float64, pin_memory=True)  # work[2:8] after the last two launches
             done = [torch.cuda.Event(), torch.cuda.Event()]
-            batch = 0
-            while k < self.pcgMaxIter:
-                step = min(10, self.pcgMaxIter - k)
-                if self.pcgGraphs and step == 10 and k >= 20:
-                    if graph is None:
-                        graph = self._capture_pcg_batch(lib, s, k, step)
-                    graph.replay()
-                else:
-                    L.check(lib.efe_pcg_iterate(ctypes.byref(s), k, step, stream), "efe_pcg_iterate")
-                k += step
-                seen[batch % 2].copy_(work[2:4], non_blocking=True)
-                done[batch % 2].record()
-                batch += 1
-                if batch < 2:
+            launched, i = 0, 0
+            while True:
+                step = min(segment, self.pcgMaxIter - launched)
+                L.check(lib.efe_pcg_solve(ctypes.byref(s), cols, asm.nnz, launched, step, 10, tol2, stream), "efe_pcg_solve")
+                launched += step
+                seen[i % 2].copy_(work[2:8], non_blocking=True)
+                done[i % 2].record()
+                i += 1
+                more = launched < self.pcgMaxIter
+                if i < 2 and more:
                     continue
-                done[batch % 2].synchronize()  # the previous batch (the one just queued still runs)
-                rr, pAp = seen[batch % 2].tolist()
-                if not rr <= tol2 and rr == rr and pAp != 0.0:  # not converged, no NaN, no breakdown
-                    continue
-                break
+                last = (i if more else i + 1) % 2  # the previous launch (the one just queued still runs), or the last one
+                done[last].synchronize()
+                ended, k = seen[last][3].item(), int(seen[last][4])
+                if ended < 0:
+                    raise RuntimeError("a wait inside the device CG gave up: the solution is invalid")
+                if ended or not more:
+                    break
         self._record_linear(k, bnorm, tol2, lambda: float(work[2]))
         return vec[0] + xd
 
@@ -513,16 +521,6 @@ class NISTGPU:
         else:
             self._record_linear(k, bnorm, tol2, lambda: 0.0)
         return x + xd
-
-    def _capture_pcg_batch(self, lib, s, k, step):
-        """One batch of `step` PCG iterations starting at iteration k (even) as a CUDA graph."""
-        import ctypes
-
-        from . import _lib as L
-
-        dev = self.asm.device
-        return self._capture(lambda: L.check(lib.efe_pcg_iterate(ctypes.byref(s), k, step, ctypes.c_void_p(
-            torch.cuda.current_stream(dev).cuda_stream)), "efe_pcg_iterate (graph capture)"))  # fmt: skip
 
     def _capture(self, fn):
         """The launches of fn() as a CUDA graph, captured on a side stream (fn launches on the

@@ -297,6 +297,16 @@ typedef struct EfePcg {
 int32_t efe_csr_spmv(const EfePcg* solver, const double* x, double* y, void* stream);
 int32_t efe_pcg_start(const EfePcg* solver, const double* b, void* stream);
 int32_t efe_pcg_iterate(const EfePcg* solver, int64_t firstIteration, int32_t nIterations, void* stream);
+/* efe_pcg_iterate with the convergence test on the device.  After every `every` iterations (counted from
+   the start of the solve) the residual is tested: the solve ends one batch of `every` iterations after
+   the first one with r.r <= tol2, a NaN or p.Ap = 0, or when nIterations have run.  work[5] then holds 1
+   if it has ended (further calls do nothing), 0 if it goes on, -1 if a wait inside the kernel gave up
+   (an internal error: the solution is invalid); work[6] the iterations run, work[2] r.r and work[3]
+   p.Ap of the last.  blockCols (optional, device): with patternBlock 2 or 3, the rows' columns also come
+   in aligned blocks of that many, and blockCols[indptr[r] / patternBlock^2 + k] is the first column of
+   block k of the row group starting at row r.  nnz: stored entries (0: not known).  */
+int32_t efe_pcg_solve(const EfePcg* solver, const int32_t* blockCols, int64_t nnz, int64_t firstIteration,
+                      int32_t nIterations, int32_t every, double tol2, void* stream);
 
 /* Building blocks of a multilevel (aggregation) preconditioner for the same systems; the reference
    reaches multilevel methods only through external solvers behind linearSolve
