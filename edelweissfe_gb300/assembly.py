@@ -59,8 +59,8 @@ class GPUAssembler:
     (-1 for nodes without DOFs; DofManager numbering, `numerics/dofmanager.py:259-300`);
     nDof: size of the DOF vectors; groups: ElementGroup list in the reference's element order.
     precision: "fp64" (everything FP64), "mixed" (FP32 tangent, FP64 residual and state) or
-    "mixed-ff" (as "mixed", with the small-strain strain increment and element residual in
-    float-float arithmetic; the return map, state and global residual accumulation stay FP64)."""
+    "mixed-ff" (as "mixed", with the kinematics and element residual of total-Lagrangian Neo-Hooke groups
+    in float-float arithmetic; the return map, state and global residual accumulation stay FP64)."""
 
     def __init__(self, coords, nodeDof, nDof, groups, precision="fp64", device=None):
         self.lib = L.load()

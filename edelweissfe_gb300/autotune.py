@@ -31,11 +31,9 @@ def variants_for(asm, gi):
 def default_variant(asm, gi):
     """Tile variant of group gi before (or without) autotuning.  The tensor-core tangent for total-
     Lagrangian Hexa20 groups (faster than the SIMT tiles in both FP32-tangent modes) and for small-
-    strain Hexa20 groups with an FP64 residual (mixed); 0 for small-strain Hexa20 groups with a
-    float-float residual (mixed-ff), where the tensor-core tile, which runs the FP64 return map of an
-    element's 27 points on one warp, is about even with the SIMT tile for linear hardening and slower
-    for saturation hardening (C3D20 J2 plastic increment, 16,384 elements: 16.7 against 17.7 M
-    elem/s)."""
+    strain Hexa20 groups in the mixed mode; 0 for small-strain Hexa20 groups in the mixed-ff mode, where
+    the tensor-core tile, which runs the FP64 return map of an element's 27 points on one warp, is about
+    even with the SIMT tile for linear hardening and slower for saturation hardening."""
     from . import _lib as L
     from .library import element_type
 

@@ -374,9 +374,27 @@ struct VMConst {
   double G, fy0, H, dfy, delta;
   double tfac;  // 1 / (1 + H / (3G)): the tangent factor of vonmises.py:247 when dfy == 0
   double invdR; // 1 / (dR/d dK) of the return-map residual, constant per element when dfy == 0
+  double sq6G, g15;  // sqrt(6) G, 2 G sqrt(1.5) (von_mises_3d_f32)
 };
+// FAST: with the FP32 tangent
+template <bool FAST = false>
 __device__ __forceinline__ VMConst vm_const(const double* props, bool vonMises) {
   VMConst c;
+  if constexpr (FAST) {  // two divisions instead of five: the same constants up to rounding
+    const double E = props[0], v = props[1], a = 1.0 + v, b = 1.0 - 2.0 * v, r = 1.0 / (a * b), f = E * r;
+    c.Ei = Iso{f * (1.0 - v), f * v, f * (b * 0.5)};
+    c.G = c.Ei.c44;
+    c.fy0 = vonMises ? props[2] : 0.0;
+    c.H = vonMises ? props[3] : 0.0;
+    c.dfy = vonMises ? props[4] : 0.0;
+    c.delta = vonMises ? props[5] : 0.0;
+    const double g3 = 3.0 * c.G, q = 1.0 / (g3 + c.H);
+    c.tfac = g3 * q;
+    c.invdR = -sqrt(1.5) * q;  // 1 / (-sqrt(2/3) (3 G + H))
+    c.sq6G = sqrt(6.0) * c.G;
+    c.g15 = 2.0 * sqrt(1.5) * c.G;
+    return c;
+  }
   c.Ei = iso3d(props[0], props[1]);
   c.G = props[0] / (2.0 * (1.0 + props[1]));
   c.fy0 = vonMises ? props[2] : 0.0;
@@ -385,6 +403,8 @@ __device__ __forceinline__ VMConst vm_const(const double* props, bool vonMises) 
   c.delta = vonMises ? props[5] : 0.0;
   c.tfac = 1.0 / (1.0 + c.H / (3.0 * c.G));
   c.invdR = 1.0 / (-sqrt(6.0) * c.G - sqrt(2.0 / 3.0) * c.H);
+  c.sq6G = sqrt(6.0) * c.G;
+  c.g15 = 2.0 * sqrt(1.5) * c.G;
   return c;
 }
 
@@ -489,15 +509,94 @@ __device__ inline bool von_mises_3d(const VMConst& c, double sig[6], const doubl
   return true;
 }
 
-__device__ __forceinline__ void linear_elastic_3d(const VMConst& c, double sig[6], const double de[6], Tangent3& T) {
-  double ds[6];
-  iso_apply(c.Ei, de, ds);
-  for (int i = 0; i < 6; ++i) sig[i] += ds[i];
-  T.c11 = c.Ei.c11;
+// The von Mises update of the FP32-tangent modes: von_mises_3d with fewer FP64 instructions (53 against 92 for linear
+// hardening).  The zero-increment test is decided in FP32 where it is clear, the trial stress is sig + lambda tr de +
+// 2 G de, and the flow direction, which only the tangent takes, is formed in FP32.
+struct TangentF32 {
+  double c12, c44, a;
+  float n[6];
+};
+__device__ inline bool von_mises_3d_f32(const VMConst& c, double sig[6], const double de[6], double& kappa, TangentF32& T) {
   T.c12 = c.Ei.c12;
   T.c44 = c.Ei.c44;
   T.a = 0.0;
-  for (int i = 0; i < 6; ++i) T.n[i] = 0.0;
+  float z = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    T.n[i] = 0.0f;
+    const float d = d2f_trunc(de[i]);
+    z = fmaf(d, d, z);
+  }
+  if (!(z > 2e-28f)) {  // near or below |dStrain| = 1e-14 (vonmises.py:211-213), or not a number
+    double nrm = 0.0;
+    for (int i = 0; i < 6; ++i) nrm += de[i] * de[i];
+    if (nrm < 1e-28) return true;
+  }
+  double tr[6], dev[6];
+  const double g2e = 2.0 * c.Ei.c44, lt = c.Ei.c12 * (de[0] + de[1] + de[2]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    tr[i] = fma(g2e, de[i], sig[i] + lt);
+    tr[3 + i] = fma(c.Ei.c44, de[3 + i], sig[3 + i]);
+  }
+  const double mean = (tr[0] + tr[1] + tr[2]) * (1.0 / 3.0);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dev[i] = tr[i] - mean;
+    dev[3 + i] = tr[3 + i];
+  }
+  const double q2 = fma(2.0, fma(dev[5], dev[5], fma(dev[4], dev[4], dev[3] * dev[3])),
+                        fma(dev[2], dev[2], fma(dev[1], dev[1], dev[0] * dev[0])));
+  const double inv = rsqrt(q2), devNorm = q2 > 0.0 ? q2 * inv : 0.0;
+  const double k0 = kappa, sq23 = sqrt(2.0 / 3.0);
+  const bool lin = c.dfy == 0.0;
+  auto residual = [&](double dK, double k) {
+    double fy = fma(c.H, k, c.fy0);
+    if (!lin) fy += vm_sat(c, k);
+    return fma(-sq23, fy, fma(-c.sq6G, dK, devNorm));
+  };
+  double R = residual(0.0, k0);
+  if (!(R > 0.0)) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) sig[i] = tr[i];
+    return true;
+  }
+  double dK = 0.0, k = k0;
+  bool ok = true;
+  for (int counter = 0; fabs(R) > 1e-12; ++counter) {
+    if (counter == 15) {
+      ok = false;
+      break;
+    }
+    dK -= vm_newton_step(c, R, k);
+    k = k0 + dK;
+    R = residual(dK, k);
+  }
+  kappa = k;
+  const double gi = c.g15 * dK * inv, beta = 2.0 * c.G * gi;
+  const float invF = ff_split_rn_bits(inv).h;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    sig[i] = fma(-gi, dev[i], tr[i]);
+    T.n[i] = ff_split_rn_bits(dev[i]).h * invF;
+  }
+  const double tfac = lin ? c.tfac : 1.0 / (1.0 + (c.H + vm_dsat(c, k)) / (3.0 * c.G));
+  T.a = 2.0 * c.G * (tfac - gi);
+  T.c12 = fma(beta, 1.0 / 3.0, c.Ei.c12);
+  T.c44 = fma(beta, -0.5, c.Ei.c44);
+  return ok;
+}
+
+template <typename TangentT>
+__device__ __forceinline__ void linear_elastic_3d(const VMConst& c, double sig[6], const double de[6], TangentT& T) {
+  double ds[6];
+  iso_apply(c.Ei, de, ds);
+  for (int i = 0; i < 6; ++i) sig[i] += ds[i];
+  if constexpr (std::is_same<TangentT, Tangent3>::value) T.c11 = c.Ei.c11;
+  T.c12 = c.Ei.c12;
+  T.c44 = c.Ei.c44;
+  T.a = 0.0;
+  for (int i = 0; i < 6; ++i) T.n[i] = 0;
 }
 
 // symmetric 3x3 in-plane tangent (rows/cols 11, 22, 12): C00 C01 C02 C11 C12 C22

@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "efe_device.cuh"
+#include "efe_fixed.cuh"
 #include "efe_tc.cuh"
 
 namespace efe {
@@ -161,7 +162,6 @@ __global__ void body_force_kernel(int64_t nSel, const int32_t* __restrict__ elem
 // ------------------------------------------------------------------ assembly
 enum Form { SS3 = 0, SS2 = 1, TLH = 2, TLV3 = 3, TLV2 = 4 };
 template <int FORM, int DIM> struct FormInfo;
-template <int DIM> struct FormInfo<SS3, DIM> { static constexpr int NVEC = 2, NSCAL = 3; };
 template <int DIM> struct FormInfo<SS2, DIM> { static constexpr int NVEC = 1, NSCAL = 6; };
 template <int DIM> struct FormInfo<TLH, DIM> { static constexpr int NVEC = 5, NSCAL = 2; };
 template <int DIM> struct FormInfo<TLV3, DIM> { static constexpr int NVEC = 4, NSCAL = 9; };
@@ -210,12 +210,35 @@ struct TCState {
 // MMA chunk takes.  On expiry the CTA records EFE_STATUS_TC_TIMEOUT and stops issuing MMAs.
 constexpr int TC_WAIT_LIMIT = 1 << 22;
 
-// FF: the strain increment and the residual of the small-strain 3D form are formed in float-float
-// arithmetic from the float-float geometry (geomG32 + geomGlo); the return map stays FP64.
+}  // namespace efe
+
+#include "efe_ss3.cuh"
+
+namespace efe {
+
+// Hexa8 2x2x2 with an FP32 tangent: warps of four elements
+template <int SHAPE, int RULE, typename KT>
+__host__ __device__ constexpr bool ss3_warp_tile() {
+  return SHAPE == EFE_HEXA8 && RULE == EFE_RULE_3D_2X2X2 && std::is_same<KT, float>::value;
+}
+
+// the tile of the small-strain solids has a layout of its own
+template <int SHAPE, int RULE, int FORM, typename KT, int EPB>
+struct LayoutOf : std::conditional<FORM == SS3, SS3Layout<ShapeInfo<SHAPE>::DIM == 3 ? SHAPE : EFE_HEXA8, RULE, KT, EPB>,
+                                   Layout<SHAPE, RULE, FORM, KT, EPB>>::type {};
+
+// FF: the deformation gradient and the residual of the total-Lagrangian Neo-Hooke form in float-float arithmetic from
+// the float-float geometry (geomG32 + geomGlo); the material update stays FP64.
 // One tile: the EPB elements starting at e0, processed by the NT threads of the calling CTA
 // (every thread of the CTA must call it: it synchronises the CTA).
 template <int SHAPE, int RULE, int FORM, typename KT, int EPB, int NT, bool FF>
 __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
+  if constexpr (FORM == SS3) {
+    if constexpr (ss3_warp_tile<SHAPE, RULE, KT>())
+      assemble_tile_ss3_hexa8<NT>(g, e0, smem);
+    else
+      assemble_tile_ss3<SHAPE, RULE, KT, EPB, NT>(g, e0, smem);
+  } else {
   using L = Layout<SHAPE, RULE, FORM, KT, EPB>;
   constexpr int DIM = L::DIM, NN = L::NN, NQ = L::NQ, NVEC = L::NVEC, NDOF = L::NDOF;
   // the faster return-map arithmetic goes with the FP32 tangent (mixed modes)
@@ -462,12 +485,10 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
     if (e >= nEl) continue;
     const int64_t pt = e * NQ + q;
     double Gm[DIM][NN];
-    if constexpr (!FF) {
 #pragma unroll
-      for (int c = 0; c < DIM; ++c)
+    for (int c = 0; c < DIM; ++c)
 #pragma unroll
-        for (int a = 0; a < NN; ++a) Gm[c][a] = g.geomG[(int64_t)(c * NN + a) * stride + pt];
-    }
+      for (int a = 0; a < NN; ++a) Gm[c][a] = g.geomG[(int64_t)(c * NN + a) * stride + pt];
     const double s = g.geomS[pt];
     const double* u = su + le * NN * DIM;
     const double* props = g.props + e * g.nProps;
@@ -483,140 +504,39 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
     const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
     if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
 
-    if constexpr (FORM == SS3 || FORM == SS2) {
+    if constexpr (FORM == SS2) {
       // ------------------------------------------------ small strain (element.py:318-346)
       double de[6] = {0, 0, 0, 0, 0, 0};
-      ff Gf[DIM][NN];
-      if constexpr (FF) {
-        const ff* uf = reinterpret_cast<const ff*>(su) + le * NN * DIM;
-        ff acc[6] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
-        for (int a = 0; a < NN; ++a) {
-          for (int c = 0; c < DIM; ++c)
-            Gf[c][a] = ff{g.geomG32[(int64_t)(c * NN + a) * stride + pt], g.geomGlo[(int64_t)(c * NN + a) * stride + pt]};
-          const ff ux = uf[a * 3 + 0], uy = uf[a * 3 + 1], uz = uf[a * 3 + 2 % DIM];
-          ff_fma(acc[0], Gf[0][a], ux);
-          ff_fma(acc[1], Gf[1][a], uy);
-          ff_fma(acc[2], Gf[2 % DIM][a], uz);
-          ff_fma(acc[3], Gf[1][a], ux);
-          ff_fma(acc[3], Gf[0][a], uy);
-          ff_fma(acc[4], Gf[2 % DIM][a], ux);
-          ff_fma(acc[4], Gf[0][a], uz);
-          ff_fma(acc[5], Gf[2 % DIM][a], uy);
-          ff_fma(acc[5], Gf[1][a], uz);
-        }
-        for (int f = 0; f < 6; ++f) de[f] = ff_to_double_bits(acc[f]);
-      } else if constexpr (DIM == 3) {
-        for (int a = 0; a < NN; ++a) {
-          const double ux = u[a * 3 + 0], uy = u[a * 3 + 1], uz = u[a * 3 + 2];
-          const double gx = Gm[0][a], gy = Gm[1][a], gz = Gm[2][a];
-          // one FMA per product (B . dU, element.py:322)
-          de[0] = fma(gx, ux, de[0]);
-          de[1] = fma(gy, uy, de[1]);
-          de[2] = fma(gz, uz, de[2]);
-          de[3] = fma(gx, uy, fma(gy, ux, de[3]));
-          de[4] = fma(gx, uz, fma(gz, ux, de[4]));
-          de[5] = fma(gy, uz, fma(gz, uy, de[5]));
-        }
-      } else {
-        for (int a = 0; a < NN; ++a) {
-          const double ux = u[a * DIM + 0], uy = u[a * DIM + 1];
-          const double gx = Gm[0][a], gy = Gm[1][DIM == 2 ? a : a];
-          de[0] += gx * ux;
-          de[1] += gy * uy;
-          de[3] += gy * ux + gx * uy;
-        }
+      for (int a = 0; a < NN; ++a) {
+        const double ux = u[a * DIM + 0], uy = u[a * DIM + 1];
+        const double gx = Gm[0][a], gy = Gm[1][a];
+        de[0] += gx * ux;
+        de[1] += gy * uy;
+        de[3] += gy * ux + gx * uy;
       }
-      if constexpr (FORM == SS3) {
+      Tangent2 C;
+      if (g.plane == EFE_PLANE_STRESS) {
+        if (g.material == EFE_MAT_VON_MISES)
+          ok = von_mises_plane_stress<FASTRM>(smc[le], sig, de, kappa, C);
+        else
+          linear_elastic_plane_stress(props, sig, de, C);
+      } else {
         Tangent3 T;
         if (g.material == EFE_MAT_VON_MISES)
           ok = von_mises_3d<FASTRM>(smc[le], sig, de, kappa, T);
         else
           linear_elastic_3d(smc[le], sig, de, T);
-        // residual r_a = s * sigma . G_a   (small-strain Voigt order 11,22,33,12,13,23)
-        if constexpr (FF) {
-          ff sf[6];
-          const ff s_ff = ff_split_bits(s);
-          for (int f = 0; f < 6; ++f) sf[f] = ff_mul(ff_split_bits(sig[f]), s_ff);
-          ff* rf = reinterpret_cast<ff*>(rq);
-          for (int a = 0; a < NN; ++a) {
-            ff r0{0, 0}, r1{0, 0}, r2{0, 0};
-            ff_fma(r0, sf[0], Gf[0][a]);
-            ff_fma(r0, sf[3], Gf[1][a]);
-            ff_fma(r0, sf[4], Gf[2 % DIM][a]);
-            ff_fma(r1, sf[3], Gf[0][a]);
-            ff_fma(r1, sf[1], Gf[1][a]);
-            ff_fma(r1, sf[5], Gf[2 % DIM][a]);
-            ff_fma(r2, sf[4], Gf[0][a]);
-            ff_fma(r2, sf[5], Gf[1][a]);
-            ff_fma(r2, sf[2], Gf[2 % DIM][a]);
-            rf[a * DIM + 0] = r0;
-            rf[a * DIM + 1] = r1;
-            rf[a * DIM + 2 % DIM] = r2;
-          }
-        } else {
-          double ss[6];
-          for (int f = 0; f < 6; ++f) ss[f] = sig[f] * s;
-          for (int a = 0; a < NN; ++a) {
-            const double gx = Gm[0][a], gy = Gm[1][a], gz = Gm[2 % DIM][a];
-            rq[a * DIM + 0] = ss[0] * gx + ss[3] * gy + ss[4] * gz;
-            rq[a * DIM + 1] = ss[3] * gx + ss[1] * gy + ss[5] * gz;
-            rq[a * DIM + 2 % DIM] = ss[4] * gx + ss[5] * gy + ss[2] * gz;
-          }
-        }
-        sc[0] = to_kt<KT>(T.c12 * s);
-        sc[1] = to_kt<KT>(T.c44 * s);
-        sc[2] = to_kt<KT>(T.a * s);
-        // tangent vectors G_a and n.G_a in the tangent's precision (FP32 copy of G when present)
-        KT n[6];
-        for (int f = 0; f < 6; ++f) n[f] = to_kt<KT>(T.n[f]);
-        for (int a = 0; a < NN; ++a) {
-          KT gx, gy, gz;
-          if constexpr (FF) {
-            gx = Gf[0][a].h;
-            gy = Gf[1][a].h;
-            gz = Gf[2 % DIM][a].h;
-          } else if (std::is_same<KT, float>::value && g.geomG32) {
-            gx = (KT)g.geomG32[(int64_t)(0 * NN + a) * stride + pt];
-            gy = (KT)g.geomG32[(int64_t)(1 * NN + a) * stride + pt];
-            gz = (KT)g.geomG32[(int64_t)(2 * NN + a) * stride + pt];
-          } else {
-            gx = (KT)Gm[0][a];
-            gy = (KT)Gm[1][a];
-            gz = (KT)Gm[2 % DIM][a];
-          }
-          KT* v = vq + a * NVEC * DIM;
-          v[0] = gx;
-          v[1] = gy;
-          v[2 % DIM] = gz;
-          v[DIM + 0] = n[0] * gx + n[3] * gy + n[4] * gz;
-          v[DIM + 1] = n[3] * gx + n[1] * gy + n[5] * gz;
-          v[DIM + 2 % DIM] = n[4] * gx + n[5] * gy + n[2] * gz;
-        }
-      } else {
-        Tangent2 C;
-        if (g.plane == EFE_PLANE_STRESS) {
-          if (g.material == EFE_MAT_VON_MISES)
-            ok = von_mises_plane_stress<FASTRM>(smc[le], sig, de, kappa, C);
-          else
-            linear_elastic_plane_stress(props, sig, de, C);
-        } else {
-          Tangent3 T;
-          if (g.material == EFE_MAT_VON_MISES)
-            ok = von_mises_3d<FASTRM>(smc[le], sig, de, kappa, T);
-          else
-            linear_elastic_3d(smc[le], sig, de, T);
-          tangent2_from3(T, C);
-        }
-        for (int a = 0; a < NN; ++a) {
-          const double gx = Gm[0][a], gy = Gm[1 % DIM][a];
-          rq[a * DIM + 0] = (sig[0] * gx + sig[3] * gy) * s;
-          rq[a * DIM + 1 % DIM] = (sig[3] * gx + sig[1] * gy) * s;
-          KT* v = vq + a * NVEC * DIM;
-          v[0] = (KT)gx;
-          v[1 % DIM] = (KT)gy;
-        }
-        for (int k = 0; k < 6; ++k) sc[k] = (KT)(C.c[k] * s);
+        tangent2_from3(T, C);
       }
+      for (int a = 0; a < NN; ++a) {
+        const double gx = Gm[0][a], gy = Gm[1 % DIM][a];
+        rq[a * DIM + 0] = (sig[0] * gx + sig[3] * gy) * s;
+        rq[a * DIM + 1 % DIM] = (sig[3] * gx + sig[1] * gy) * s;
+        KT* v = vq + a * NVEC * DIM;
+        v[0] = (KT)gx;
+        v[1 % DIM] = (KT)gy;
+      }
+      for (int k = 0; k < 6; ++k) sc[k] = (KT)(C.c[k] * s);
       for (int f = 0; f < 6; ++f) eps[f] += de[f];
     } else {
       // ------------------------------------------------ total Lagrangian (displacementtlelement/element.py:346-427)
@@ -800,16 +720,7 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
       const KT* sc = ssc + (le * NQ + q) * L::SC;
       const KT* va = sv + (size_t)(le * NQ + q) * L::SV + a * NVEC * DIM;
       const KT* vb = sv + (size_t)(le * NQ + q) * L::SV + b * NVEC * DIM;
-      if constexpr (FORM == SS3) {
-        const KT Lq = sc[0], Mq = sc[1], Aq = sc[2];
-        const KT dot = va[0] * vb[0] + va[1] * vb[1] + va[2 % DIM] * vb[2 % DIM];
-#pragma unroll
-        for (int j = 0; j < DIM; ++j)
-#pragma unroll
-          for (int k = 0; k < DIM; ++k)
-            acc[j][k] += Lq * va[j] * vb[k] + Mq * ((j == k ? dot : KT(0)) + va[k] * vb[j]) -
-                         Aq * va[DIM + j] * vb[DIM + k];
-      } else if constexpr (FORM == SS2) {
+      if constexpr (FORM == SS2) {
         // B columns (11,22,12): (a,0) = [gx, 0, gy], (a,1) = [0, gy, gx]
         const KT c00 = sc[0], c01 = sc[1], c02 = sc[2], c11 = sc[3], c12 = sc[4], c22 = sc[5];
         const KT ax = va[0], ay = va[1 % DIM], bx = vb[0], by = vb[1 % DIM];
@@ -903,6 +814,7 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
 #pragma unroll
         for (int k = 0; k < DIM; ++k) kadd(K + slot2 + (int64_t)j * rl2 + k, acc[j][k]);
     }
+  }
   }
 }
 

@@ -10,13 +10,13 @@ namespace efe {
 // thread in phase A), 128 threads, at most 72 KB of shared memory so that three CTAs share an SM.
 // Variant 1: about 256 points and 256 threads per CTA, up to 110 KB (one or two CTAs per SM).
 // The autotuner (edelweissfe_gb300/autotune.py) picks one per group by timing both.
-template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT = 0>
-struct Tile {
+template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT>
+struct TileOf {
   // variant 0: 128 threads, ~128 points, 3 CTAs/SM where they fit; 1: 256 threads, ~256 points;
   // 2: variant 0's tile with 4 CTAs/SM where shared memory allows (the compiler then holds the
   // kernel to 128 registers per thread)
   static constexpr int NQ = RuleInfo<RULE>::NQ;
-  static constexpr size_t per_element = Layout<SHAPE, RULE, FORM, KT, 1>::bytes;
+  static constexpr size_t per_element = LayoutOf<SHAPE, RULE, FORM, KT, 1>::bytes;
   static constexpr size_t budget = VARIANT == 1 ? 110 * 1024 : 72 * 1024;
   static constexpr int points = VARIANT == 1 ? 256 : 128;
   static constexpr int fit = (int)(budget / per_element);
@@ -24,11 +24,21 @@ struct Tile {
   static constexpr int e0 = fit < want ? fit : want;
   static constexpr int EPB = e0 < 1 ? 1 : (e0 > 32 ? 32 : e0);
   static constexpr int NT = VARIANT == 1 ? 256 : 128;
-  static constexpr size_t bytes = Layout<SHAPE, RULE, FORM, KT, EPB>::bytes;
+  static constexpr size_t bytes = LayoutOf<SHAPE, RULE, FORM, KT, EPB>::bytes;
   static constexpr int MINB = VARIANT == 1 ? 1
                               : (VARIANT == 2 && bytes <= 56 * 1024) ? 4
                               : (bytes <= 72 * 1024 ? 3 : 1);
 };
+// The warp tile of small-strain Hexa8 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: six CTAs of
+// four warps per SM hold the kernel to 80 registers (40 B of spills); five CTAs (96 registers) or four (128) run in 1.01
+// and 1.06 times its time on 262144 elements, 1.00 and 1.05 times on 65231.
+struct WarpTile {
+  static constexpr int NT = 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = 6;
+  static constexpr size_t bytes = SS3Hexa8Layout<NT>::bytes;
+};
+template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT = 0>
+struct Tile : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile,
+                               TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type {};
 
 template <int SHAPE, int RULE, int FORM, typename KT, bool FF, int VARIANT>
 cudaError_t launch_assemble_variant(const GroupArgs& g, cudaStream_t st) {
@@ -105,11 +115,16 @@ cudaError_t launch_assemble(const GroupArgs& g, cudaStream_t st) {
   if constexpr (has_tc_variant<SHAPE, RULE, FORM, KT>()) {
     if (g.tileVariant == 3) return launch_assemble_tc<FF, FORM>(g, st);
   }
-  if (g.tileVariant == 1) return launch_assemble_variant<SHAPE, RULE, FORM, KT, FF, 1>(g, st);
+  // the small-strain solids' SIMT tile forms its B-products in integers in either mode
+  constexpr bool ffTile = FF && FORM != SS3;
+  // Small-strain Hexa20 with an FP32 tangent takes the wide shape in any case: its phases with a thread per point fill
+  // eight warps, not the 81 points of three elements four of them (602 against 653 us on 13824 elements, von Mises)
+  constexpr bool wide = SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && FORM == SS3 && std::is_same<KT, float>::value;
+  if (wide || g.tileVariant == 1) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 1>(g, st);
   if constexpr (Tile<SHAPE, RULE, FORM, KT, 2>::MINB != Tile<SHAPE, RULE, FORM, KT, 0>::MINB) {
-    if (g.tileVariant == 2) return launch_assemble_variant<SHAPE, RULE, FORM, KT, FF, 2>(g, st);
+    if (g.tileVariant == 2) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 2>(g, st);
   }
-  return launch_assemble_variant<SHAPE, RULE, FORM, KT, FF, 0>(g, st);
+  return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 0>(g, st);
 }
 
 template <int SHAPE, int RULE>

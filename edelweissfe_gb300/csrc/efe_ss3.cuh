@@ -1,0 +1,653 @@
+// efe_ss3.cuh -- the small-strain solid element pass (von Mises, linear elastic; Hexa8, Hexa20) with its
+// B-products in fixed-point integers (efe_fixed.cuh); included by efe_kernels.cuh.
+//
+// What is left to the FP64 pipe, which bound this pass in every mode, is the material update (92 instructions per point,
+// 53 with an FP32 tangent).  The strain increment de = B dU (9 products per node and point), the residual
+// s B^T sigma (9 again) and, with an FP64 tangent, the element stiffness (27 per node pair and point) are sums
+// over few terms of one scale per element, so they run as integer multiply-adds and are exact apart from the
+// rounding of the operands.
+//
+// Scales (biased exponents): dN/dX of a point em_g, the element's dU em_u, over the element's points of s sigma
+// times the point's dN/dX em_s, of the tangent's coefficients (c12 s and c44 s; a s) times dN/dX twice em_c, em_a: the
+// per-point factors are rounded relative to em_s - em_g, em_c - 2 em_g and em_a - 2 em_g, so that all points of a sum
+// share one scale.
+//
+// Measured, von Mises plastic increment, kernel time before (FP64 sums) and with integers: C3D8, FP64 tangent, 31713
+// elements 1027 -> 362 us; FP32 tangent, 262144 elements 1318 -> 995 us; C3D20, FP64 tangent, 2448 elements 1638 -> 325
+// us; FP32 tangent, 13824 elements 954 -> 599 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
+// -> 2.2e-15, K 7.2e-16 -> 7.1e-16; C3D20 P 5.4e-15 -> 5.3e-15, K 1.89e-15 -> 1.88e-15; FP32 K 6.1e-8 in both.
+//
+// FP64 tangent: K_ab = sum_q  c12 s G_a (x) G_b + c44 s (G_b (x) G_a + G_a . G_b I) - a s nG_a (x) nG_b.  The
+// operands c12 s G, c44 s G, -a s nG and nG of every point and node are formed once (integer products of the
+// digits); a node pair then takes 27 products per point.
+#pragma once
+
+namespace efe {
+
+template <int SHAPE, int RULE, typename KT, int EPB>
+struct SS3Layout {
+  static constexpr int DIM = 3, NN = ShapeInfo<SHAPE>::NN, NQ = RuleInfo<RULE>::NQ, NDOF = 3 * NN, NP = EPB * NQ;
+  static constexpr bool F64 = std::is_same<KT, double>::value;
+  // odd strides per point: consecutive points fall on different banks
+  static constexpr int GS = NDOF | 1, SV = (2 * NDOF) | 1, DS = 7;
+  static constexpr size_t u_off = 0;                                         // double, then fx [EPB][NDOF]
+  static constexpr size_t g_off = u_off + 8 * EPB * NDOF;                    // fx [NP][GS]: dN/dX
+  static constexpr size_t d_off = g_off + 8 * NP * GS;                       // [NP][DS]: strain, then s sigma (double, fx)
+  static constexpr size_t k_off = d_off + 8 * NP * DS;                       // F64: fx [4][NP][GS], else KT [NP][SV]
+  // flow direction n: double, then fx (F64), or float where the tangent's vectors are formed per point and node
+  static constexpr size_t n_off = (k_off + (F64 ? (size_t)32 * NP * GS : (size_t)4 * NP * SV) + 7) / 8 * 8;  // [NP][DS]
+  static constexpr size_t c_off = (n_off + (F64 || NN > 8 || NQ > 8 ? sizeof(KT) * NP * DS : 0) + 7) / 8 * 8;  // KT [NP][3]: coefficients
+  static constexpr size_t mc_off = (c_off + sizeof(KT) * NP * 3 + 15) / 16 * 16;  // VMConst [EPB]
+  static constexpr size_t rl_off = mc_off + sizeof(VMConst) * EPB;                // int [EPB][NN]
+  static constexpr size_t e_off = rl_off + sizeof(int) * EPB * NN;                // int [EPB]: em_u, em_s, em_c, em_a; [NP]: em_g
+  static constexpr size_t bytes = e_off + sizeof(int) * (4 * EPB + NP);
+};
+
+__device__ __forceinline__ int fx_max_exponent(int em, double x) { return max(em, fx_exponent(x)); }
+
+template <int SHAPE, int RULE, typename KT, int EPB, int NT>
+__device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
+  using L = SS3Layout<SHAPE, RULE, KT, EPB>;
+  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, GS = L::GS, SV = L::SV, DS = L::DS;
+  constexpr bool F64 = L::F64;
+  // one thread forms a point's digits and strain where a point has few nodes (the tile has a thread per point)
+  constexpr bool PERPOINT = NN == 8 && NP <= NT;
+  double* su = reinterpret_cast<double*>(smem + L::u_off);
+  fx* suf = reinterpret_cast<fx*>(smem + L::u_off);
+  fx* sg = reinterpret_cast<fx*>(smem + L::g_off);
+  double* sd = reinterpret_cast<double*>(smem + L::d_off);
+  fx* sdf = reinterpret_cast<fx*>(smem + L::d_off);
+  KT* sv = reinterpret_cast<KT*>(smem + L::k_off);
+  fx* sset = reinterpret_cast<fx*>(smem + L::k_off);
+  KT* sn = reinterpret_cast<KT*>(smem + L::n_off);
+  fx* snf = reinterpret_cast<fx*>(smem + L::n_off);
+  KT* sc = reinterpret_cast<KT*>(smem + L::c_off);
+  fx* scf = reinterpret_cast<fx*>(smem + L::c_off);
+  VMConst* smc = reinterpret_cast<VMConst*>(smem + L::mc_off);
+  int* srl = reinterpret_cast<int*>(smem + L::rl_off);
+  int* emu = reinterpret_cast<int*>(smem + L::e_off);
+  int *ems = emu + EPB, *emc = ems + EPB, *ema = emc + EPB, *emg = ema + EPB;
+  const int tid = threadIdx.x;
+  const int64_t nEl = g.nElements, stride = nEl * NQ;
+  const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB, np = nLoc * NQ;
+
+  // ---- dU relative to the element's first node (sum_a dN_a/dX = 0), row lengths, material constants, dN/dX
+  for (int t = tid; t < 4 * EPB + NP; t += NT) emu[t] = 0;
+  if (!PERPOINT) __syncthreads();
+  double G[PERPOINT ? 3 : 1][PERPOINT ? NN : 1];
+  if constexpr (PERPOINT) {
+    if (tid < np) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int a = 0; a < NN; ++a) G[c][a] = g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + tid];
+    }
+  } else {
+    for (int t = tid; t < np * NN; t += NT) {
+      const int a = t / np, r = t - a * np;
+      int em = 0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) em = fx_max_exponent(em, g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + r]);
+      atomicMax(emg + r, em);
+    }
+  }
+  for (int t = tid; t < nLoc * NN; t += NT) {
+    const int le = t / NN, a = t - le * NN;
+    const int64_t e = e0 + le;
+    double* u = su + le * NDOF + a * 3;
+    u[0] = u[1] = u[2] = 0.0;
+    const int32_t node = g.conn[e * NN + a], node0 = g.conn[e * NN];
+    if (!in_bounds(g, node, g.nNodes, e) || !in_bounds(g, node0, g.nNodes, e)) continue;
+    srl[le * NN + a] = g.nodeRowLen[node];
+    const int32_t dof = g.nodeDof[node], dof0 = g.nodeDof[node0];
+    if (!in_bounds(g, dof, g.nDof - 2, e) || !in_bounds(g, dof0, g.nDof - 2, e)) continue;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) u[c] = g.dU[dof + c] - g.dU[dof0 + c];
+  }
+  // the last warp, which has the least of the gather
+  for (int le = NT - 1 - tid; le < nLoc; le += NT)
+    smc[le] = vm_const<!F64>(g.props + (e0 + le) * g.nProps, g.material == EFE_MAT_VON_MISES);
+  __syncthreads();
+  for (int t = tid; t < nLoc * NDOF; t += NT) atomicMax(emu + t / NDOF, fx_exponent(su[t]));
+  int eg = 0;
+  if constexpr (PERPOINT) {
+    if (tid < np) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int a = 0; a < NN; ++a) eg = fx_max_exponent(eg, G[c][a]);
+      emg[tid] = eg;
+    }
+  }
+  __syncthreads();
+
+  // ---- digits of dU and dN/dX; the FP32 tangent's dN/dX
+  for (int t = tid; t < nLoc * NDOF; t += NT) suf[t] = fx_make(su[t], emu[t / NDOF]);
+  if constexpr (PERPOINT) {
+    if (tid < np) {
+#pragma unroll
+      for (int a = 0; a < NN; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          sg[tid * GS + a * 3 + c] = fx_make(G[c][a], eg);
+          if constexpr (!F64) sv[tid * SV + a * 6 + c] = ff_split_rn_bits(G[c][a]).h;
+        }
+    }
+  } else {
+    for (int t = tid; t < np * NN; t += NT) {
+      const int a = t / np, r = t - a * np;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double x = g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + r];
+        sg[r * GS + a * 3 + c] = fx_make(x, emg[r]);
+        if constexpr (!F64) sv[r * SV + a * 6 + c] = ff_split_rn_bits(x).h;
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- strain increment (element.py:322), Voigt 11, 22, 33, 12, 13, 23 with engineering shears
+  double de[6] = {0, 0, 0, 0, 0, 0};
+  if constexpr (PERPOINT) {
+    if (tid < np) {
+      const fx* gp = sg + tid * GS;
+      const fx* up = suf + tid / NQ * NDOF;
+      FxSum s[6] = {};
+#pragma unroll
+      for (int a = 0; a < NN; ++a) {
+        const fx gx = gp[a * 3], gy = gp[a * 3 + 1], gz = gp[a * 3 + 2];
+        const fx ux = up[a * 3], uy = up[a * 3 + 1], uz = up[a * 3 + 2];
+        fx_fma(s[0], gx, ux);
+        fx_fma(s[1], gy, uy);
+        fx_fma(s[2], gz, uz);
+        fx_fma(s[3], gy, ux);
+        fx_fma(s[3], gx, uy);
+        fx_fma(s[4], gz, ux);
+        fx_fma(s[4], gx, uz);
+        fx_fma(s[5], gz, uy);
+        fx_fma(s[5], gy, uz);
+      }
+#pragma unroll
+      for (int f = 0; f < 6; ++f) de[f] = fx_value(fx_int(s[f]), eg + emu[tid / NQ]);
+    }
+  } else {
+    for (int t = tid; t < np * 6; t += NT) {
+      const int f = t / np, r = t - f * np;
+      const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+      const fx* gp = sg + r * GS;
+      const fx* up = suf + r / NQ * NDOF;
+      FxSum s{0, 0}, s2{0, 0};
+      for (int a = 0; a < NN; ++a) {
+        fx_fma(s, gp[a * 3 + j], up[a * 3 + i]);
+        if (f >= 3) fx_fma(s2, gp[a * 3 + i], up[a * 3 + j]);
+      }
+      sd[r * DS + f] = fx_value(fx_int(s, -1) + fx_int(s2, -1), emg[r] + emu[r / NQ] + 1);
+    }
+    __syncthreads();
+  }
+
+  // ---- material points (a thread per point): state, s sigma, the tangent's coefficients and flow direction
+  for (int t = tid; t < np; t += NT) {
+    const int le = t / NQ;
+    const int64_t e = e0 + le, pt = e0 * NQ + t;
+    const double s = g.geomS[pt];
+    double sig[6], eps[6], kappa = 0.0;
+    for (int f = 0; f < 6; ++f) {
+      sig[f] = g.stateRef[(int64_t)f * stride + pt];
+      eps[f] = g.stateRef[(int64_t)(6 + f) * stride + pt];
+    }
+    const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
+    if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
+    if constexpr (!PERPOINT)
+      for (int f = 0; f < 6; ++f) de[f] = sd[t * DS + f];
+    bool ok = true;
+    typename std::conditional<F64, Tangent3, TangentF32>::type T;
+    if (g.material == EFE_MAT_LINEAR_ELASTIC)
+      linear_elastic_3d(smc[le], sig, de, T);
+    else if constexpr (F64)
+      ok = von_mises_3d<false>(smc[le], sig, de, kappa, T);
+    else
+      ok = von_mises_3d_f32(smc[le], sig, de, kappa, T);
+    bool finite = true;
+    int es = 0;
+    for (int f = 0; f < 6; ++f) {
+      g.stateTemp[(int64_t)f * stride + pt] = sig[f];
+      g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
+      finite = finite && finite_bits(sig[f]);
+      const double ss = sig[f] * s;
+      sd[t * DS + f] = ss;
+      es = fx_max_exponent(es, ss);
+    }
+    if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
+    if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
+    if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
+    atomicMax(ems + le, es + emg[t]);
+    const double c[3] = {T.c12 * s, T.c44 * s, T.a * s};
+    if constexpr (F64) {
+      for (int f = 0; f < 6; ++f) sn[t * DS + f] = T.n[f];
+      for (int k = 0; k < 3; ++k) sc[t * 3 + k] = c[k];
+      int ea = fx_exponent(c[2]);
+      for (int f = 0; f < 6; ++f)
+        if (fx_exponent(T.n[f]) >= FX_NAN) ea = FX_NAN;
+      atomicMax(emc + le, max(fx_exponent(c[0]), fx_exponent(c[1])) + 2 * emg[t]);
+      atomicMax(ema + le, ea + 2 * emg[t]);
+    } else {
+      for (int k = 0; k < 3; ++k) sc[t * 3 + k] = ff_split_rn_bits(c[k]).h;
+      const float* n = T.n;
+      if constexpr (PERPOINT) {
+        for (int a = 0; a < NN; ++a) {
+          KT* v = sv + t * SV + a * 6;
+          const KT gx = v[0], gy = v[1], gz = v[2];
+          v[3] = n[0] * gx + n[3] * gy + n[4] * gz;
+          v[4] = n[3] * gx + n[1] * gy + n[5] * gz;
+          v[5] = n[4] * gx + n[5] * gy + n[2] * gz;
+        }
+      } else {
+        for (int f = 0; f < 6; ++f) sn[t * DS + f] = n[f];
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- digits of the per-point factors
+  for (int t = tid; t < np * 6; t += NT) {
+    const int r = t / 6, i = r * DS + (t - r * 6);
+    sdf[i] = fx_make(sd[i], ems[r / NQ] - emg[r]);
+    if constexpr (F64) snf[i] = fx_make(sn[i], 1023);
+  }
+  if constexpr (F64) {
+    for (int t = tid; t < np * 3; t += NT) {
+      const int r = t / 3;
+      scf[t] = fx_make(sc[t], (t - r * 3 == 2 ? ema : emc)[r / NQ] - 2 * emg[r]);
+    }
+  }
+  if constexpr (F64 || !PERPOINT) {
+    if constexpr (F64) __syncthreads();
+    // the tangent's operands per point and node
+    for (int t = tid; t < np * NN; t += NT) {
+      const int a = t / np, r = t - a * np;
+      if constexpr (F64) {
+        const fx gx = sg[r * GS + a * 3], gy = sg[r * GS + a * 3 + 1], gz = sg[r * GS + a * 3 + 2];
+        const fx* n = snf + r * DS;
+        FxSum z[3] = {};
+        fx_fma(z[0], n[0], gx);
+        fx_fma(z[0], n[3], gy);
+        fx_fma(z[0], n[4], gz);
+        fx_fma(z[1], n[3], gx);
+        fx_fma(z[1], n[1], gy);
+        fx_fma(z[1], n[5], gz);
+        fx_fma(z[2], n[4], gx);
+        fx_fma(z[2], n[5], gy);
+        fx_fma(z[2], n[2], gz);
+        const fx c0 = scf[r * 3], c1 = scf[r * 3 + 1], c2 = scf[r * 3 + 2];
+        fx* v = sset + (size_t)r * GS + a * 3;
+        const fx gv[3] = {gx, gy, gz};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const fx zc = fx_split(fx_int(z[c], -1));  // scale em_g + 1: |n| <= 1, the row of n at most 1 long
+          v[c] = fx_mul(c0, gv[c]);
+          v[(size_t)NP * GS + c] = fx_mul(c1, gv[c]);
+          v[(size_t)2 * NP * GS + c] = fx_mul(c2, zc);
+          v[(size_t)3 * NP * GS + c] = zc;
+        }
+      } else {
+        const KT* n = sn + r * DS;
+        KT* v = sv + r * SV + a * 6;
+        const KT gx = v[0], gy = v[1], gz = v[2];
+        v[3] = n[0] * gx + n[3] * gy + n[4] * gz;
+        v[4] = n[3] * gx + n[1] * gy + n[5] * gz;
+        v[5] = n[4] * gx + n[5] * gy + n[2] * gz;
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- residual and flux (NIST.computeElements, nonlinearimplicitstatic.py:837-844): P_e[a][c] = -sum_q s sigma[c] . G_a
+  for (int t = tid; t < nLoc * NDOF; t += NT) {
+    const int le = t / NDOF, k = t - le * NDOF, a = k / 3, c = k - 3 * a;
+    const int64_t e = e0 + le;
+    const int v0 = c == 0 ? 0 : c + 2, v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
+    constexpr int R = NQ > 8 ? -2 : 0;
+    FxSum s[3] = {};  // one for each direction: 27 products at most
+    for (int q = 0; q < NQ; ++q) {
+      const fx* gp = sg + (le * NQ + q) * GS + a * 3;
+      const fx* dp = sdf + (le * NQ + q) * DS;
+      fx_fma(s[0], dp[v0], gp[0]);
+      fx_fma(s[1], dp[v1], gp[1]);
+      fx_fma(s[2], dp[v2], gp[2]);
+    }
+    const double pe = -fx_value(fx_int(s[0], R) + fx_int(s[1], R) + fx_int(s[2], R), ems[le] - R);
+    const int32_t node = g.conn[e * NN + a];
+    if (!in_bounds(g, node, g.nNodes, e)) continue;
+    const int32_t dof = g.nodeDof[node] + c;
+    if (!in_bounds(g, dof, g.nDof, e)) continue;
+    atomicAdd(g.P + dof, pe);
+    atomicAdd(g.F + dof, fabs(pe));
+  }
+
+  // ---- tangent blocks of the node pairs a <= b (the element tangents are symmetric), each scattered twice
+  KT* K = reinterpret_cast<KT*>(g.Kdata);
+  constexpr int NPAIR = NN * (NN + 1) / 2;
+  for (int t = tid; t < nLoc * NPAIR; t += NT) {
+    const int le = t / NPAIR;
+    int r = t - le * NPAIR, a = 0;
+    while (r >= NN - a) {
+      r -= NN - a;
+      ++a;
+    }
+    const int b = a + r;
+    const int64_t e = e0 + le;
+    KT acc[3][3];
+    if constexpr (F64) {
+      FxSum s1[3][3] = {}, s2[3][3] = {}, s3[3][3] = {};
+#pragma unroll 1
+      for (int q = 0; q < NQ; ++q) {
+        const fx* va = sset + (size_t)(le * NQ + q) * GS + a * 3;
+        const fx* zb = sset + (size_t)(3 * NP + le * NQ + q) * GS + b * 3;
+        const fx* gb = sg + (le * NQ + q) * GS + b * 3;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const fx la = va[j], ma = va[(size_t)NP * GS + j], ta = va[(size_t)2 * NP * GS + j];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            fx_fma(s1[j][k], la, gb[k]);
+            fx_fma(s2[j][k], ma, gb[k]);
+            fx_fma(s3[j][k], ta, zb[k]);
+          }
+        }
+      }
+      // The first two sums in units of em_c - 1022, the third of em_a - 1022 + 2, added at the coarser of the two with
+      // B guard bits: as many as the largest of the 27 sums leaves (six of them add up)
+      int top = 0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) top |= fx_bits(s1[j][k]) | fx_bits(s2[j][k]) | fx_bits(s3[j][k]);
+      const int B = min(__clz(top) - 5, 26);
+      const int64_t dot = fx_int(s2[0][0], B) + fx_int(s2[1][1], B) + fx_int(s2[2][2], B);
+      const int ec = emc[le] - 1022, ea = ema[le] - 1020, d = ea - ec;
+      const int em = emc[le] >= FX_NAN || ema[le] >= FX_NAN ? FX_NAN : max(ec, ea) - B;
+      const int dc = min(max(d, 0), 63), da = min(max(-d, 0), 63);
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          acc[j][k] = fx_value(fx_shift(fx_int(s1[j][k], B) + fx_int(s2[k][j], B) + (j == k ? dot : 0), dc) -
+                                   fx_shift(fx_int(s3[j][k], B), da), em);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[j][k] = KT(0);
+      for (int q = 0; q < NQ; ++q) {
+        const KT* cq = sc + (le * NQ + q) * 3;
+        const KT* va = sv + (le * NQ + q) * SV + a * 6;
+        const KT* vb = sv + (le * NQ + q) * SV + b * 6;
+        const KT Lq = cq[0], Mq = cq[1], Aq = cq[2];
+        const KT dot = va[0] * vb[0] + va[1] * vb[1] + va[2] * vb[2];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            acc[j][k] += Lq * va[j] * vb[k] + Mq * ((j == k ? dot : KT(0)) + va[k] * vb[j]) - Aq * va[3 + j] * vb[3 + k];
+      }
+    }
+    // Ke[(a,j),(b,k)] -> CSR (row = dof(b,k), col = dof(a,j)) = slot(a,b) + k*rowLen(b) + j
+    const int32_t slot = g.pairSlot[(e * NN + a) * NN + b];
+    const int rl = srl[le * NN + b];
+    if (!in_bounds(g, slot, g.nnz, e) || !in_bounds(g, slot + (int64_t)2 * (rl + 1), g.nnz, e)) continue;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) kadd(K + slot + (int64_t)k * rl + j, acc[j][k]);
+    if (a != b) {  // Ke[(b,k),(a,j)] = Ke[(a,j),(b,k)] -> (row = dof(a,j), col = dof(b,k))
+      const int32_t slot2 = g.pairSlot[(e * NN + b) * NN + a];
+      const int rl2 = srl[le * NN + a];
+      if (!in_bounds(g, slot2, g.nnz, e) || !in_bounds(g, slot2 + (int64_t)2 * (rl2 + 1), g.nnz, e)) continue;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) kadd(K + slot2 + (int64_t)j * rl2 + k, acc[j][k]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Hexa8 with 2x2x2 points and an FP32 tangent: a warp works on four elements, a lane per point, the eight lanes of an
+// element also holding its eight nodes.  The scales are maxima and the residual a transposing sum over eight lanes;
+// the point's row of shared memory holds the digits of dN/dX and then, in their place, the tangent's vectors.  The only
+// wait for other warps is for the elements' material constants (FP64 divisions, formed by one warp for all).  262144
+// elements: 995 us; latency of the chain through a warp's phases binds it (the FP64
+// pipe is about half busy), hence few registers and 24 warps per SM.
+template <int NT>
+struct SS3Hexa8Layout {
+  static constexpr int NW = NT / 32, EPB = 4 * NW;
+  // a point's row in doublewords: 24 digits of dN/dX, then the floats (dN/dX, n dN/dX) of 8 nodes; 3 coefficients; 27,
+  // odd, so that consecutive points fall on different banks
+  static constexpr int SV = 27;
+  static constexpr size_t v_off = 0;                                            // fx [NW][32][SV]
+  static constexpr size_t u_off = v_off + sizeof(fx) * NW * 32 * SV;            // fx [NW][4][24]
+  static constexpr size_t mc_off = (u_off + sizeof(fx) * NW * 96 + 15) / 16 * 16;  // VMConst [EPB]
+  static constexpr size_t rl_off = mc_off + sizeof(VMConst) * EPB;              // int [NW][32]
+  static constexpr size_t bytes = rl_off + sizeof(int) * NW * 32;
+};
+
+template <int NT>
+__device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
+  using L = SS3Hexa8Layout<NT>;
+  constexpr int NN = 8, NQ = 8, SV = L::SV;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, le = lane >> 3, q = lane & 7;
+  fx* sv = reinterpret_cast<fx*>(smem + L::v_off) + wid * 32 * SV;
+  fx* su = reinterpret_cast<fx*>(smem + L::u_off) + wid * 96;
+  VMConst* smc = reinterpret_cast<VMConst*>(smem + L::mc_off);
+  int* srl = reinterpret_cast<int*>(smem + L::rl_off) + wid * 32;
+  float* K = reinterpret_cast<float*>(g.Kdata);
+  const int64_t nEl = g.nElements, stride = nEl * NQ, eS = e0 + wid * 4, e = eS + le, pt = eS * NQ + lane;
+  const bool vm = g.material == EFE_MAT_VON_MISES, live = e < nEl;
+  fx* row = sv + lane * SV;
+  if (wid == L::NW - 1 && lane < L::EPB && e0 + lane < nEl) smc[lane] = vm_const<true>(g.props + (e0 + lane) * g.nProps, vm);
+
+  // ---- the node's dU relative to the element's first node, digits of it and of the point's dN/dX
+  int32_t dof = -1;
+  int eg = 0, eu = 0;
+  {
+    double u[3] = {0.0, 0.0, 0.0};
+    int rl = 0;
+    if (live) {
+      const int32_t node = g.conn[e * NN + q];
+      if (in_bounds(g, node, g.nNodes, e)) {
+        rl = g.nodeRowLen[node];
+        const int32_t d = g.nodeDof[node];
+        if (in_bounds(g, d, g.nDof - 2, e)) {
+          dof = d;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) u[c] = g.dU[d + c];
+        }
+      }
+      double G[3][NN];
+      const double* gp = g.geomG + pt;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int a = 0; a < NN; ++a) G[c][a] = gp[(int64_t)(c * NN + a) * stride];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int a = 0; a < NN; ++a) eg = fx_max_exponent(eg, G[c][a]);
+#pragma unroll
+      for (int a = 0; a < NN; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) row[a * 3 + c] = fx_make(G[c][a], eg);
+    }
+    srl[lane] = rl;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      u[c] -= __shfl_sync(0xffffffffu, u[c], lane & 24);
+      eu = fx_max_exponent(eu, u[c]);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) eu = max(eu, __shfl_xor_sync(0xffffffffu, eu, o));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) su[lane * 3 + c] = fx_make(u[c], eu);
+  }
+  __syncthreads();
+
+  // ---- strain increment (element.py:322), material update, state
+  int es = 0, ep = 0;  // scales of s sigma (times dN/dX), of sigma
+  double sig[6] = {0, 0, 0, 0, 0, 0}, s = 0.0;
+  float n[6], cf[3];
+  if (live) {
+    s = g.geomS[pt];
+    double de[6], kappa = 0.0;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) sig[f] = g.stateRef[(int64_t)f * stride + pt];
+    const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
+    if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
+    {
+      FxSum acc[6] = {};
+      const fx* up = su + le * 24;
+#pragma unroll
+      for (int a = 0; a < NN; ++a) {
+        const fx ux = up[a * 3], uy = up[a * 3 + 1], uz = up[a * 3 + 2];
+        const fx gx = row[a * 3], gy = row[a * 3 + 1], gz = row[a * 3 + 2];
+        fx_fma(acc[0], gx, ux);
+        fx_fma(acc[1], gy, uy);
+        fx_fma(acc[2], gz, uz);
+        fx_fma(acc[3], gy, ux);
+        fx_fma(acc[3], gx, uy);
+        fx_fma(acc[4], gz, ux);
+        fx_fma(acc[4], gx, uz);
+        fx_fma(acc[5], gz, uy);
+        fx_fma(acc[5], gy, uz);
+      }
+#pragma unroll
+      for (int f = 0; f < 6; ++f) de[f] = fx_value(fx_int(acc[f]), eg + eu);
+    }
+    bool ok = true;
+    TangentF32 T;
+    const VMConst& mc = smc[wid * 4 + le];
+    if (vm)
+      ok = von_mises_3d_f32(mc, sig, de, kappa, T);
+    else
+      linear_elastic_3d(mc, sig, de, T);
+    bool finite = true;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      g.stateTemp[(int64_t)f * stride + pt] = sig[f];
+      g.stateTemp[(int64_t)(6 + f) * stride + pt] = g.stateRef[(int64_t)(6 + f) * stride + pt] + de[f];
+      finite = finite && finite_bits(sig[f]);
+      ep = fx_max_exponent(ep, sig[f]);
+      n[f] = T.n[f];
+    }
+    if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
+    if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
+    if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
+    es = ep + fx_exponent(s) - 1022 + eg;
+    cf[0] = ff_split_rn_bits(T.c12 * s).h;
+    cf[1] = ff_split_rn_bits(T.c44 * s).h;
+    cf[2] = ff_split_rn_bits(T.a * s).h;
+  }
+  // ---- residual: s sigma . G_a of the point for every node, summed over the element's points by exchanges that leave
+  // node q's three sums in lane q
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) es = max(es, __shfl_xor_sync(0xffffffffu, es, o));
+  {
+    const fx sd = fx_make(s, es - eg - ep + 1022);  // s sigma at the scale es - eg
+    fx d[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) d[f] = fx_mul(fx_make(sig[f], ep), sd);  // zero in lanes without a point
+    auto force = [&](int a, int c) {
+      FxSum r{0, 0};
+      fx_fma(r, d[c == 0 ? 0 : c + 2], row[a * 3]);
+      fx_fma(r, d[c == 0 ? 3 : (c == 1 ? 1 : 5)], row[a * 3 + 1]);
+      fx_fma(r, d[c == 0 ? 4 : (c == 1 ? 5 : 2)], row[a * 3 + 2]);
+      return (long long)fx_int(r);
+    };
+    if (!live)
+#pragma unroll
+      for (int k = 0; k < 24; ++k) row[k] = fx{0, 0};
+    const bool b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+    double pe[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      long long t[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const long long lo = force(a, c), hi = force(a + 4, c);
+        t[a] = (b2 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 4);
+      }
+      const long long x0 = (b1 ? t[2] : t[0]) + __shfl_xor_sync(0xffffffffu, b1 ? t[0] : t[2], 2);
+      const long long x1 = (b1 ? t[3] : t[1]) + __shfl_xor_sync(0xffffffffu, b1 ? t[1] : t[3], 2);
+      pe[c] = -fx_value((b0 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b0 ? x0 : x1, 1), es);
+    }
+    if (dof >= 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        atomicAdd(g.P + dof + c, pe[c]);
+        atomicAdd(g.F + dof + c, fabs(pe[c]));
+      }
+    }
+  }
+  // ---- the tangent's vectors in the place of the digits: the upper digit has 29 bits, more than a float
+  if (live) {
+    const float sc = eg >= FX_NAN ? __int_as_float(0x7fc00000) : (float)scalbn(1.0, max(-300, min(300, eg - 1051)));
+#pragma unroll
+    for (int a = 0; a < NN; ++a) {
+      const float gx = (float)row[a * 3].h * sc, gy = (float)row[a * 3 + 1].h * sc, gz = (float)row[a * 3 + 2].h * sc;
+      float2* v = reinterpret_cast<float2*>(row + a * 3);
+      v[0] = make_float2(gx, gy);
+      v[1] = make_float2(gz, n[0] * gx + n[3] * gy + n[4] * gz);
+      v[2] = make_float2(n[3] * gx + n[1] * gy + n[5] * gz, n[4] * gx + n[5] * gy + n[2] * gz);
+    }
+    float2* v = reinterpret_cast<float2*>(row + 24);
+    v[0] = make_float2(cf[0], cf[1]);
+    v[1] = make_float2(cf[2], 0.0f);
+  }
+  __syncwarp();
+
+  // ---- tangent: the 36 node pairs as (a, a + d mod 8), d = 0 .. 3 for every a and d = 4 for a < 4
+  const int nLoc = nEl - eS < 4 ? (int)(nEl - eS) : 4;
+  for (int t = lane; t < nLoc * 36; t += 32) {
+    const int el = t / 36, r = t - el * 36, a = r & 7, b = (a + (r >> 3)) & 7;
+    const int64_t ee = eS + el;
+    const int32_t slot = g.pairSlot[(ee * NN + a) * NN + b], slot2 = g.pairSlot[(ee * NN + b) * NN + a];
+    float acc[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, dot = 0.0f;
+    const float2* base = reinterpret_cast<const float2*>(sv + el * NQ * SV);
+#pragma unroll 2
+    for (int p = 0; p < NQ; ++p) {
+      const float2 *va = base + p * SV + a * 3, *vb = base + p * SV + b * 3, *cq = base + p * SV + 24;
+      const float2 a0 = va[0], a1 = va[1], a2 = va[2], b0 = vb[0], b1 = vb[1], b2 = vb[2], c0 = cq[0], c1 = cq[1];
+      const float ga[3] = {a0.x, a0.y, a1.x}, na[3] = {a1.y, a2.x, a2.y};
+      const float gb[3] = {b0.x, b0.y, b1.x}, nb[3] = {b1.y, b2.x, b2.y};
+      float lg[3], mg[3], tn[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        lg[j] = c0.x * ga[j];
+        mg[j] = c0.y * ga[j];
+        tn[j] = -c1.x * na[j];
+        dot = fmaf(mg[j], gb[j], dot);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[j][k] = fmaf(tn[j], nb[k], fmaf(mg[k], gb[j], fmaf(lg[j], gb[k], acc[j][k])));
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) acc[j][j] += dot;
+    // Ke[(a,j),(b,k)] -> CSR (row = dof(b,k), col = dof(a,j)) = slot(a,b) + k*rowLen(b) + j, and its transpose
+    const int rb = srl[el * NN + b], ra = srl[el * NN + a];
+    if (!in_bounds(g, slot, g.nnz, ee) || !in_bounds(g, slot + (int64_t)2 * (rb + 1), g.nnz, ee)) continue;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) kadd(K + slot + (int64_t)k * rb + j, acc[j][k]);
+    if (a == b) continue;
+    if (!in_bounds(g, slot2, g.nnz, ee) || !in_bounds(g, slot2 + (int64_t)2 * (ra + 1), g.nnz, ee)) continue;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) kadd(K + slot2 + (int64_t)j * ra + k, acc[j][k]);
+  }
+}
+
+}  // namespace efe

@@ -73,9 +73,10 @@ enum {
   EFE_K_FP64 = 0, /* everything in FP64 (Kdata is double*)                                   */
   EFE_K_FP32 = 1, /* tangent formed and accumulated in FP32 (Kdata is float*); residual, state
                      and the return map stay FP64                                              */
-  EFE_K_FP32_FF = 2 /* as EFE_K_FP32, and for small-strain solids the strain increment and the
-                     element residual, for total-Lagrangian Neo-Hooke F, F^-T dN/dX and the
-                     element residual are formed in float-float arithmetic (~48-bit significand,
+  EFE_K_FP32_FF = 2 /* as EFE_K_FP32, and for total-Lagrangian Neo-Hooke F, F^-T dN/dX and the
+                     element residual (on tile variant 3 also the small-strain solids' strain
+                     increment and element residual, which otherwise are exact integer sums in
+                     every mode) are formed in float-float arithmetic (~48-bit significand,
                      needs geomG32 and geomGlo); the return map / Kirchhoff stress, state and the
                      global residual accumulation stay FP64                                    */
 };
