@@ -9,13 +9,13 @@ import os
 import torch
 
 VARIANTS = (0, 1, 2)
-TENSOR_VARIANT = 3  # the element tangent on the tensor cores (Hexa20 3x3x3 TL Neo-Hooke or small strain, FP32 tangent)
+TENSOR_VARIANT = 3  # the element tangent on the tensor cores (Hexa20 3x3x3 TL Neo-Hooke, FP32 tangent)
 
 
 def variants_for(asm, gi):
     """Tile variants to time for group gi: the CTA shapes 0-2, and the tensor-core tangent where the
-    library has it (Hexa20 3x3x3, total-Lagrangian with a hyperelastic material or small strain,
-    with an FP32 tangent)."""
+    library has it (Hexa20 3x3x3, total-Lagrangian with a hyperelastic material, with an FP32
+    tangent; small-strain Hexa20 takes the number too and runs its one SIMT tile under each)."""
     from . import _lib as L
     from .library import element_type
 
@@ -29,11 +29,9 @@ def variants_for(asm, gi):
 
 
 def default_variant(asm, gi):
-    """Tile variant of group gi before (or without) autotuning.  The tensor-core tangent for total-
-    Lagrangian Hexa20 groups (faster than the SIMT tiles in both FP32-tangent modes) and for small-
-    strain Hexa20 groups in the mixed mode; 0 for small-strain Hexa20 groups in the mixed-ff mode, where
-    the tensor-core tile, which runs the FP64 return map of an element's 27 points on one warp, is about
-    even with the SIMT tile for linear hardening and slower for saturation hardening."""
+    """Tile variant of group gi before (or without) autotuning: the tensor-core tangent for total-
+    Lagrangian Hexa20 groups (faster than the SIMT tiles in both FP32-tangent modes), else 0.  Small-
+    strain Hexa20 groups run the same tile under every number."""
     from . import _lib as L
     from .library import element_type
 

@@ -222,6 +222,12 @@ __host__ __device__ constexpr bool ss3_warp_tile() {
   return SHAPE == EFE_HEXA8 && RULE == EFE_RULE_3D_2X2X2 && std::is_same<KT, float>::value;
 }
 
+// Hexa20 3x3x3 with an FP32 tangent: two elements on four warps
+template <int SHAPE, int RULE, typename KT>
+__host__ __device__ constexpr bool ss3_hexa20_tile() {
+  return SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && std::is_same<KT, float>::value;
+}
+
 // the tile of the small-strain solids has a layout of its own
 template <int SHAPE, int RULE, int FORM, typename KT, int EPB>
 struct LayoutOf : std::conditional<FORM == SS3, SS3Layout<ShapeInfo<SHAPE>::DIM == 3 ? SHAPE : EFE_HEXA8, RULE, KT, EPB>,
@@ -236,6 +242,8 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
   if constexpr (FORM == SS3) {
     if constexpr (ss3_warp_tile<SHAPE, RULE, KT>())
       assemble_tile_ss3_hexa8<NT>(g, e0, smem);
+    else if constexpr (ss3_hexa20_tile<SHAPE, RULE, KT>())
+      assemble_tile_ss3_hexa20(g, e0, smem);
     else
       assemble_tile_ss3<SHAPE, RULE, KT, EPB, NT>(g, e0, smem);
   } else {
@@ -851,12 +859,11 @@ __device__ __forceinline__ void tc_end(TCState& tcs) {
   if (threadIdx.x < 32) tc::tmem_dealloc(tcs.tmem, H20TC::TMEM_COLS);
 }
 
-// Tile variant 3, the Hexa20 3x3x3 pass (total-Lagrangian Neo-Hooke or small strain) with the
-// tensor-core tangent (efe_hexa20_tc.cuh): a grid of resident CTAs (sms per wave), one element per tile, tiles strided by
+// Tile variant 3, the Hexa20 3x3x3 total-Lagrangian Neo-Hooke pass with the tensor-core tangent (efe_hexa20_tc.cuh): a grid of resident CTAs (sms per wave), one element per tile, tiles strided by
 // the grid; each CTA allocates its TMEM columns once and frees them at the end.  The CTAs of one
 // wave share no SM, so the wave index picks the warp of the per-point update.  Each element's
 // K_e scatter runs during the next element's material update (the last one after the loop).
-template <bool FF, int FORM>
+template <bool FF>
 __global__ void __launch_bounds__(128, 3) assemble_kernel_tc(GroupArgs g, int sms) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t mbar;
@@ -866,7 +873,7 @@ __global__ void __launch_bounds__(128, 3) assemble_kernel_tc(GroupArgs g, int sm
   int64_t prev = H20TC_DEFER_NONE;  // the element whose K_e is pending in shared memory
   for (int64_t e = blockIdx.x; e < g.nElements; e += gridDim.x, ++rot, par ^= 1) {
     const int64_t next = e + gridDim.x < g.nElements ? e + gridDim.x : -1;
-    assemble_tile_h20tc<FF, FORM>(g, e, smem, tcs, rot, prev, next, prev >= 0, par);
+    assemble_tile_h20tc<FF>(g, e, smem, tcs, rot, prev, next, prev >= 0, par);
     prev = e;
     __syncthreads();
   }
@@ -922,7 +929,7 @@ __device__ __forceinline__ bool persistent_tile(const GroupTables<N>& tabs, long
     int k = 0;
     while (t >= tb.tileStart[k + 1]) ++k;
     if constexpr (T0::TC)
-      assemble_tile_h20tc<FF, T0::FORM>(tb.g[k], (int64_t)(t - tb.tileStart[k]), smem, *tcs, rot, H20TC_NOW, -1, false,
+      assemble_tile_h20tc<FF>(tb.g[k], (int64_t)(t - tb.tileStart[k]), smem, *tcs, rot, H20TC_NOW, -1, false,
                                           0);
     else
       assemble_tile<T0::SHAPE, T0::RULE, T0::FORM, KT, T0::EPB, NT, FF>(tb.g[k], (int64_t)(t - tb.tileStart[k]) * T0::EPB,

@@ -36,9 +36,16 @@ struct WarpTile {
   static constexpr int NT = 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = 6;
   static constexpr size_t bytes = SS3Hexa8Layout<NT>::bytes;
 };
+// The two-element tile of small-strain Hexa20 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: five CTAs per
+// SM (96 registers); four (128) or six (80, 116 B of spills) run in 1.06 and 1.07 times its time.
+struct Hexa20Tile {
+  static constexpr int NT = SS3Hexa20Layout::NT, EPB = SS3Hexa20Layout::EPB, MINB = 5;
+  static constexpr size_t bytes = SS3Hexa20Layout::bytes;
+};
 template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT = 0>
 struct Tile : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile,
-                               TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type {};
+                               typename std::conditional<FORM == SS3 && ss3_hexa20_tile<SHAPE, RULE, KT>(), Hexa20Tile,
+                                                         TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type>::type {};
 
 template <int SHAPE, int RULE, int FORM, typename KT, bool FF, int VARIANT>
 cudaError_t launch_assemble_variant(const GroupArgs& g, cudaStream_t st) {
@@ -53,12 +60,13 @@ cudaError_t launch_assemble_variant(const GroupArgs& g, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// the tensor-core tangent (tile variant 3) exists for the Hexa20 3x3x3 total-Lagrangian Neo-Hooke
-// and small-strain (von Mises, linear elastic) forms with an FP32 tangent
+// the tensor-core tangent (tile variant 3) exists for the Hexa20 3x3x3 total-Lagrangian Neo-Hooke form with an FP32
+// tangent; on small-strain Hexa20 variant 3 names the two-element tile too, which runs in 372 us where a tensor-core tile
+// took 678 (13824 elements, von Mises): its FP64 return map on one warp at a time and its twelve warps per SM
+// bound that one
 template <int SHAPE, int RULE, int FORM, typename KT>
 constexpr bool has_tc_variant() {
-  return SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && (FORM == TLH || FORM == SS3) &&
-         std::is_same<KT, float>::value;
+  return SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && FORM == TLH && std::is_same<KT, float>::value;
 }
 
 // Resident CTAs per SM of a kernel that allocates tmemCols TMEM columns per CTA, from its registers
@@ -87,12 +95,12 @@ cudaError_t resident_ctas_tmem(K kern, int nt, size_t dynBytes, int tmemCols, in
   return n >= 1 ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
-template <bool FF, int FORM>
+template <bool FF>
 cudaError_t launch_assemble_tc(const GroupArgs& g, cudaStream_t st) {
   constexpr int NT = 128;
   constexpr size_t bytes = H20TCLayout<FF>::bytes;
   static_assert(bytes <= 74 * 1024, "three tensor-core tiles must fit in one SM");
-  auto kern = assemble_kernel_tc<FF, FORM>;
+  auto kern = assemble_kernel_tc<FF>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   // the largest shared-memory partition: without it the occupancy query (and the launch) assume the
@@ -112,15 +120,11 @@ cudaError_t launch_assemble_tc(const GroupArgs& g, cudaStream_t st) {
 
 template <int SHAPE, int RULE, int FORM, typename KT, bool FF = false>
 cudaError_t launch_assemble(const GroupArgs& g, cudaStream_t st) {
+  constexpr bool ffTile = FF && FORM != SS3;  // the small-strain solids form their B-products in integers in either mode
   if constexpr (has_tc_variant<SHAPE, RULE, FORM, KT>()) {
-    if (g.tileVariant == 3) return launch_assemble_tc<FF, FORM>(g, st);
+    if (g.tileVariant == 3) return launch_assemble_tc<FF>(g, st);
   }
-  // the small-strain solids' SIMT tile forms its B-products in integers in either mode
-  constexpr bool ffTile = FF && FORM != SS3;
-  // Small-strain Hexa20 with an FP32 tangent takes the wide shape in any case: its phases with a thread per point fill
-  // eight warps, not the 81 points of three elements four of them (602 against 653 us on 13824 elements, von Mises)
-  constexpr bool wide = SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && FORM == SS3 && std::is_same<KT, float>::value;
-  if (wide || g.tileVariant == 1) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 1>(g, st);
+  if (g.tileVariant == 1) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 1>(g, st);
   if constexpr (Tile<SHAPE, RULE, FORM, KT, 2>::MINB != Tile<SHAPE, RULE, FORM, KT, 0>::MINB) {
     if (g.tileVariant == 2) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 2>(g, st);
   }

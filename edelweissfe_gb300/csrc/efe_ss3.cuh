@@ -14,7 +14,7 @@
 //
 // Measured, von Mises plastic increment, kernel time before (FP64 sums) and with integers: C3D8, FP64 tangent, 31713
 // elements 1027 -> 362 us; FP32 tangent, 262144 elements 1318 -> 995 us; C3D20, FP64 tangent, 2448 elements 1638 -> 325
-// us; FP32 tangent, 13824 elements 954 -> 599 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
+// us; FP32 tangent, 13824 elements 678 -> 372 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
 // -> 2.2e-15, K 7.2e-16 -> 7.1e-16; C3D20 P 5.4e-15 -> 5.3e-15, K 1.89e-15 -> 1.88e-15; FP32 K 6.1e-8 in both.
 //
 // FP64 tangent: K_ab = sum_q  c12 s G_a (x) G_b + c44 s (G_b (x) G_a + G_a . G_b I) - a s nG_a (x) nG_b.  The
@@ -531,10 +531,13 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
     else
       linear_elastic_3d(mc, sig, de, T);
     bool finite = true;
+    // all loads before the first store, which they could not pass
+#pragma unroll
+    for (int f = 0; f < 6; ++f) de[f] += g.stateRef[(int64_t)(6 + f) * stride + pt];
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
       g.stateTemp[(int64_t)f * stride + pt] = sig[f];
-      g.stateTemp[(int64_t)(6 + f) * stride + pt] = g.stateRef[(int64_t)(6 + f) * stride + pt] + de[f];
+      g.stateTemp[(int64_t)(6 + f) * stride + pt] = de[f];
       finite = finite && finite_bits(sig[f]);
       ep = fx_max_exponent(ep, sig[f]);
       n[f] = T.n[f];
@@ -647,6 +650,332 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
     for (int j = 0; j < 3; ++j)
 #pragma unroll
       for (int k = 0; k < 3; ++k) kadd(K + slot2 + (int64_t)j * ra + k, acc[j][k]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Hexa20 with 3x3x3 points and an FP32 tangent: two elements on four warps.  A point's row of shared memory holds the
+// digits of dN/dX and then, in their place, the tangent's vectors; a thread forms the blocks of 2 x 2 nodes (14 loads of
+// shared memory for 138 arithmetic instructions per point), and K_e goes to the CSR rows through shared memory, so that
+// the lanes of a warp share the sectors that L2 adds to (the adds alone: 110 us on 13824 elements, 264 us by node pairs).
+// 372 us; the issue slots (63 % used) and the waits of the phases with a thread per point bind it.
+struct SS3Hexa20Layout {
+  static constexpr int EPB = 2, NT = 128, NN = 20, NQ = 27, NDOF = 60, NP = EPB * NQ, NB = 55;  // NB: node blocks A <= B
+  // a point's row in doublewords: 60 digits, then the floats (dN/dX, n dN/dX) of 20 nodes; odd
+  static constexpr int SV = 61, DS = 7, SK = 61;
+  static constexpr size_t v_off = 0;                            // fx [NP][SV]
+  static constexpr size_t u_off = v_off + 8 * NP * SV;          // fx [EPB][NDOF]
+  static constexpr size_t d_off = u_off + 8 * EPB * NDOF;       // int64 [NP][DS]: half of the strain; fx: s sigma
+  static constexpr size_t k_bytes = 4 * EPB * NDOF * SK;        // K_e, in their place: float [EPB][NDOF][SK]
+  static_assert(k_bytes <= d_off + 8 * NP * DS, "K_e fits the area of the operands");
+  static constexpr size_t c_off = (d_off + 8 * NP * DS + 15) / 16 * 16;  // float4 [NP]: coefficients, unit of the upper digits
+  static constexpr size_t n_off = c_off + 16 * NP;              // float [NP][DS]: flow direction
+  static constexpr size_t mc_off = (n_off + 4 * NP * DS + 15) / 16 * 16;  // VMConst [EPB]
+  static constexpr size_t sl_off = mc_off + sizeof(VMConst) * EPB;        // int [EPB][NN][NN]: pair slots
+  static constexpr size_t rl_off = sl_off + 4 * EPB * NN * NN;            // int [EPB][NN]: row lengths
+  static constexpr size_t e_off = rl_off + 4 * EPB * NN;                  // int [2][NP]: halves of em_g; [EPB]: em_u, em_s
+  static constexpr size_t bytes = e_off + 4 * (2 * NP + 2 * EPB);
+};
+
+__device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
+  using L = SS3Hexa20Layout;
+  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, SV = L::SV, DS = L::DS, EPB = L::EPB, NT = L::NT;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  fx* sv = reinterpret_cast<fx*>(smem + L::v_off);
+  fx* su = reinterpret_cast<fx*>(smem + L::u_off);
+  int64_t* sde = reinterpret_cast<int64_t*>(smem + L::d_off);
+  fx* sd = reinterpret_cast<fx*>(smem + L::d_off);
+  float4* sc = reinterpret_cast<float4*>(smem + L::c_off);
+  float* sn = reinterpret_cast<float*>(smem + L::n_off);
+  VMConst* smc = reinterpret_cast<VMConst*>(smem + L::mc_off);
+  int* sps = reinterpret_cast<int*>(smem + L::sl_off);
+  int* srl = reinterpret_cast<int*>(smem + L::rl_off);
+  int* sem = reinterpret_cast<int*>(smem + L::e_off);
+  int *emu = sem + 2 * NP, *ems = emu + EPB;
+  const int64_t nEl = g.nElements, stride = nEl * NQ;
+  const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB;
+  const bool vm = g.material == EFE_MAT_VON_MISES;
+
+  for (int t = tid; t < nLoc * NN * NN; t += NT) tc::cp_async4(sps + t, g.pairSlot + e0 * NN * NN + t);
+  // ---- dN/dX: two threads per point, 30 values each; dU relative to the element's first node: warps 0 and 1; the
+  // material constants: two lanes of warp 3 that have no points
+  {
+    const int part = tid / NP, r = tid - part * NP;
+    const bool live = part < 2 && r < nLoc * NQ;
+    constexpr int H = NDOF / 2;
+    double G[H];
+    int em = 0;
+    if (live) {
+      const double* gp = g.geomG + (int64_t)(part * H) * stride + e0 * NQ + r;
+#pragma unroll
+      for (int i = 0; i < H; ++i) G[i] = gp[(int64_t)i * stride];
+    }
+    const int le = wid;
+    if (le < EPB) {
+      double u[3] = {0.0, 0.0, 0.0};
+      int eu = 0;
+      const int64_t e = e0 + le;
+      if (lane < NN && le < nLoc) {
+        const int32_t node = g.conn[e * NN + lane], node0 = g.conn[e * NN];
+        int rl = 0;
+        if (in_bounds(g, node, g.nNodes, e) && in_bounds(g, node0, g.nNodes, e)) {
+          rl = g.nodeRowLen[node];
+          const int32_t dof = g.nodeDof[node], dof0 = g.nodeDof[node0];
+          if (in_bounds(g, dof, g.nDof - 2, e) && in_bounds(g, dof0, g.nDof - 2, e)) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              u[c] = g.dU[dof + c] - g.dU[dof0 + c];
+              eu = fx_max_exponent(eu, u[c]);
+            }
+          }
+        }
+        srl[le * NN + lane] = rl;
+      }
+      eu = __reduce_max_sync(0xffffffffu, eu);
+      if (lane < NN)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) su[le * NDOF + lane * 3 + c] = fx_make(u[c], eu);
+      if (lane == 0) emu[le] = eu;
+    }
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < H; ++i) em = fx_max_exponent(em, G[i]);
+      sem[part * NP + r] = em;
+    }
+    if (wid == 3 && lane >= 32 - nLoc) {
+      const int k = 31 - lane;
+      smc[k] = vm_const<true>(g.props + (e0 + k) * g.nProps, vm);
+    }
+    __syncthreads();
+    if (live) {
+      em = max(sem[r], sem[NP + r]);
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const int la = part * H + i, c = la / NN, a = la - c * NN;
+        sv[r * SV + a * 3 + c] = fx_make(G[i], em);
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- strain increment (element.py:322): two warps per element, a lane per point, ten nodes each
+  const int le = wid >> 1, half = wid & 1, pr = le * NQ + lane;
+  const bool live = le < nLoc && lane < NQ;
+  const int eg = live ? max(sem[pr], sem[NP + pr]) : 0;
+  const int64_t e = e0 + le, pt = e * NQ + lane;
+  const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
+  int64_t st[6];
+  double sig[6], kappa = 0.0, s = 0.0;
+  if (live && half == 0) {
+#pragma unroll
+    for (int f = 0; f < 6; ++f) sig[f] = g.stateRef[(int64_t)f * stride + pt];
+    if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
+    s = g.geomS[pt];
+  }
+  if (live) {
+    FxSum acc[6] = {};
+    const fx *gp = sv + pr * SV + half * 30, *up = su + le * NDOF + half * 30;
+#pragma unroll 5
+    for (int a = 0; a < NN / 2; ++a) {
+      const fx ux = up[a * 3], uy = up[a * 3 + 1], uz = up[a * 3 + 2];
+      const fx gx = gp[a * 3], gy = gp[a * 3 + 1], gz = gp[a * 3 + 2];
+      fx_fma(acc[0], gx, ux);
+      fx_fma(acc[1], gy, uy);
+      fx_fma(acc[2], gz, uz);
+      fx_fma(acc[3], gy, ux);
+      fx_fma(acc[3], gx, uy);
+      fx_fma(acc[4], gz, ux);
+      fx_fma(acc[4], gx, uz);
+      fx_fma(acc[5], gz, uy);
+      fx_fma(acc[5], gy, uz);
+    }
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      st[f] = fx_int(acc[f], -1);
+      if (half) sde[pr * DS + f] = st[f];
+    }
+  }
+  __syncthreads();
+
+  // ---- material points: one warp of each element
+  if (half == 0) {
+    int es = 0;
+    double ss[6] = {0, 0, 0, 0, 0, 0};
+    if (live) {
+      double de[6], eps[6];
+#pragma unroll
+      for (int f = 0; f < 6; ++f) {
+        de[f] = fx_value(st[f] + sde[pr * DS + f], eg + emu[le] + 1);
+        eps[f] = g.stateRef[(int64_t)(6 + f) * stride + pt];
+      }
+      bool ok = true;
+      TangentF32 T;
+      if (vm)
+        ok = von_mises_3d_f32(smc[le], sig, de, kappa, T);
+      else
+        linear_elastic_3d(smc[le], sig, de, T);
+      bool finite = true;
+#pragma unroll
+      for (int f = 0; f < 6; ++f) {
+        g.stateTemp[(int64_t)f * stride + pt] = sig[f];
+        g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
+        finite = finite && finite_bits(sig[f]);
+        ss[f] = s * sig[f];
+        es = fx_max_exponent(es, ss[f]);
+        sn[pr * DS + f] = T.n[f];
+      }
+      if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
+      if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
+      if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
+      // the upper digits of dN/dX have 29 bits, more than a float
+      const float unit = eg >= FX_NAN ? __int_as_float(0x7fc00000) : ldexpf(1.0f, max(-300, min(300, eg - 1051)));
+      sc[pr] = make_float4(ff_split_rn_bits(T.c12 * s).h, ff_split_rn_bits(T.c44 * s).h, ff_split_rn_bits(T.a * s).h, unit);
+      es += eg;
+    }
+    es = __reduce_max_sync(0xffffffffu, es);
+    if (lane == 0) ems[le] = es;
+    if (live)
+#pragma unroll
+      for (int f = 0; f < 6; ++f) sd[pr * DS + f] = fx_make(ss[f], es - eg);
+  }
+  __syncthreads();
+
+  // ---- residual and flux (NIST.computeElements, nonlinearimplicitstatic.py:837-844): 60 threads per element
+  {
+    const int el = tid >> 6, k = tid & 63;
+    if (k < NDOF && el < nLoc) {
+      const int a = k / 3, c = k - 3 * a;
+      const int64_t e = e0 + el;
+      const int v0 = c == 0 ? 0 : c + 2, v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
+      FxSum s[3] = {};  // one for each direction: 27 products
+      const fx *gp = sv + el * NQ * SV + a * 3, *dp = sd + el * NQ * DS;
+#pragma unroll 3
+      for (int q = 0; q < NQ; ++q) {
+        fx_fma(s[0], dp[q * DS + v0], gp[q * SV]);
+        fx_fma(s[1], dp[q * DS + v1], gp[q * SV + 1]);
+        fx_fma(s[2], dp[q * DS + v2], gp[q * SV + 2]);
+      }
+      const double pe = -fx_value(fx_int(s[0], -2) + fx_int(s[1], -2) + fx_int(s[2], -2), ems[el] + 2);
+      const int32_t node = g.conn[e * NN + a];
+      if (in_bounds(g, node, g.nNodes, e)) {
+        const int32_t dof = g.nodeDof[node] + c;
+        if (in_bounds(g, dof, g.nDof, e)) {
+          atomicAdd(g.P + dof, pe);
+          atomicAdd(g.F + dof, fabs(pe));
+        }
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- the tangent's vectors in the place of the digits
+  if (live) {
+    const float unit = sc[pr].w;
+    float n[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) n[f] = sn[pr * DS + f];
+    fx* row = sv + pr * SV + half * 30;
+#pragma unroll 5
+    for (int a = 0; a < NN / 2; ++a) {
+      const float gx = (float)row[a * 3].h * unit, gy = (float)row[a * 3 + 1].h * unit, gz = (float)row[a * 3 + 2].h * unit;
+      float2* v = reinterpret_cast<float2*>(row + a * 3);
+      v[0] = make_float2(gx, gy);
+      v[1] = make_float2(gz, n[0] * gx + n[3] * gy + n[4] * gz);
+      v[2] = make_float2(n[3] * gx + n[1] * gy + n[5] * gz, n[4] * gx + n[5] * gy + n[2] * gz);
+    }
+  }
+  __syncthreads();
+
+  // ---- tangent: blocks of the nodes (2A, 2A + 1) x (2B, 2B + 1), A <= B, 64 threads per element
+  const int el = tid >> 6;
+  int B = tid & 63, A = 0;
+  const bool has = B < L::NB && el < nLoc;
+  float acc[2][2][3][3] = {};
+  if (has) {
+    while (B >= NN / 2 - A) {
+      B -= NN / 2 - A;
+      ++A;
+    }
+    B += A;
+    float dot[2][2] = {};
+    const float2* base = reinterpret_cast<const float2*>(sv + el * NQ * SV);
+#pragma unroll 1
+    for (int q = 0; q < NQ; ++q) {
+      float ga[2][3], na[2][3], gb[2][3], nb[2][3];
+      const float4 c = sc[el * NQ + q];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const float2 *va = base + q * SV + (2 * A + x) * 3, *vb = base + q * SV + (2 * B + x) * 3;
+        const float2 a0 = va[0], a1 = va[1], a2 = va[2], b0 = vb[0], b1 = vb[1], b2 = vb[2];
+        ga[x][0] = a0.x, ga[x][1] = a0.y, ga[x][2] = a1.x, na[x][0] = a1.y, na[x][1] = a2.x, na[x][2] = a2.y;
+        gb[x][0] = b0.x, gb[x][1] = b0.y, gb[x][2] = b1.x, nb[x][0] = b1.y, nb[x][1] = b2.x, nb[x][2] = b2.y;
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float lg[3], mg[3], tn[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          lg[j] = c.x * ga[x][j];
+          mg[j] = c.y * ga[x][j];
+          tn[j] = -c.z * na[x][j];
+        }
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            dot[x][y] = fmaf(mg[j], gb[y][j], dot[x][y]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              acc[x][y][j][k] += fmaf(tn[j], nb[y][k], fmaf(mg[k], gb[y][j], lg[j] * gb[y][k]));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) acc[x][y][j][j] += dot[x][y];
+  }
+  tc::cp_async_wait_all();
+  __syncthreads();
+
+  // ---- K_e[(b, k)][(a, j)] over the operands (the element tangents are symmetric), then a warp per node b: its three
+  // CSR rows, 30 lanes for the columns (a, j) of ten nodes: slot(a, b) + k rowLen(b) + j
+  float* sK = reinterpret_cast<float*>(smem) + el * NDOF * L::SK;
+  if (has) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int ca = (2 * A + x) * 3 + j, cb = (2 * B + y) * 3 + k;
+            sK[cb * L::SK + ca] = acc[x][y][j][k];
+            if (A != B) sK[ca * L::SK + cb] = acc[x][y][j][k];
+          }
+  }
+  __syncthreads();
+  {
+    float* K = reinterpret_cast<float*>(g.Kdata);
+    const int a0 = lane / 3, j = lane - 3 * a0;
+    if (lane < 30) {
+      for (int t = wid; t < nLoc * NN; t += NT / 32) {
+        const int m = t / NN, b = t - m * NN, rl = srl[m * NN + b];
+        const int64_t e = e0 + m;
+        const float* row = reinterpret_cast<const float*>(smem) + (m * NDOF + 3 * b) * L::SK;
+#pragma unroll
+        for (int a = a0; a < NN; a += 10) {
+          const int32_t slot = sps[(m * NN + a) * NN + b];
+          if (!in_bounds(g, slot, g.nnz, e) || !in_bounds(g, slot + (int64_t)2 * (rl + 1), g.nnz, e)) continue;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) atomicAdd(K + slot + (int64_t)k * rl + j, row[k * L::SK + 3 * a + j]);
+        }
+      }
+    }
   }
 }
 

@@ -74,11 +74,10 @@ enum {
   EFE_K_FP32 = 1, /* tangent formed and accumulated in FP32 (Kdata is float*); residual, state
                      and the return map stay FP64                                              */
   EFE_K_FP32_FF = 2 /* as EFE_K_FP32, and for total-Lagrangian Neo-Hooke F, F^-T dN/dX and the
-                     element residual (on tile variant 3 also the small-strain solids' strain
-                     increment and element residual, which otherwise are exact integer sums in
-                     every mode) are formed in float-float arithmetic (~48-bit significand,
-                     needs geomG32 and geomGlo); the return map / Kirchhoff stress, state and the
-                     global residual accumulation stay FP64                                    */
+                     element residual are formed in float-float arithmetic (~48-bit significand,
+                     needs geomG32 and geomGlo); the Kirchhoff stress, state and the global
+                     residual accumulation stay FP64 (small-strain solids form their strain and
+                     residual in exact integer sums in every mode)                              */
 };
 /* status words (int32[3], zeroed by the caller): status[0] = OR of EFE_STATUS_* bits,
    status[1] = INT32_MAX - (global index of the first failing element), 0 if none,
