@@ -14,15 +14,21 @@
 // With gX, also the adjoint of the nodal coordinates: per point, G = dN/dX enters de = B dU and
 // the residual, s = det J w t the residual; Gbar_a = sym(deBar) u_a - s sigma PBar_a and
 // sBar = -sigma : (B PBar), and through G = J^-1 D (D = J G, J = D' X with the Hexa20 quirk row in
-// D'): Xbar_a = -M^T G_a + s sBar G_a (+ the quirk row's term), M = sum_a Gbar_a (x) G_a.
+// D'): Xbar_a = -M^T G_a + s sBar G_a (+ the quirk row's term), M = sum_a Gbar_a (x) G_a = sym(deBar) Hu -
+// s sigma Hp with the gradients Hu of dU and Hp of PBar.
 //
 // Plane stress (2D): the reverse of the reference's local Newton on eps33, iteration by iteration.
 //
 // Tile: EPB elements per CTA.  Phase 0 gathers dU_e and PBar_e, stages the tile's dN/dX rows in
 // shared memory (cp.async) and forms the elements' constants once; phase A runs one thread per
 // point (B dU, B PBar, the reverse update, the point's strain adjoint); phase C forms B^T deBar per
-// element DOF over the points (one atomic per element DOF) and sums the property adjoints (plain
-// stores: one thread owns an element's property).
+// element DOF over the points (one atomic per element DOF), likewise the coordinate adjoint, and sums the property
+// adjoints (plain stores: one thread owns an element's property).
+//
+// Measured, before (FP64 or float-float sums, the coordinate adjoint node by node and point by point) and now: C3D20,
+// 6912 elements 218 -> 211 us (the reverse return map keeps the FP64 pipe half busy with eleven warps per SM, which
+// shared memory bounds); C3D20 fp64, 1728 elements 110 -> 65 us, with gX 319 -> 189; C3D8, 32768 elements 208 -> 190 us, with
+// gX 518 -> 350.
 #pragma once
 #include "efe_launch.cuh"
 
@@ -39,18 +45,31 @@ struct SSRevConst {
   double rDR;       // 1 / (sqrt(6) G + sqrt(2/3) H): minus the return map's Newton factor (linear hardening)
   double r3G;       // 1 / (3 G)
 };
+// four divisions, independent of one another but for the last
 __device__ inline SSRevConst ss_rev_const(const double* props, bool vonMises) {
   SSRevConst r;
-  r.c = vm_const(props, vonMises);
   r.E = props[0];
   r.nu = props[1];
+  const double n1 = 1.0 + r.nu, n2 = 1.0 - 2.0 * r.nu;
   r.rE = 1.0 / r.E;
-  r.r1nu = 1.0 / (1.0 + r.nu);
-  const double rden = 1.0 / ((1.0 + r.nu) * (1.0 - 2.0 * r.nu));
+  r.r1nu = 1.0 / n1;
+  const double rden = r.r1nu * (1.0 / n2);
   r.f = r.E * rden;
-  r.df = r.E * (1.0 + 4.0 * r.nu) * rden * rden;
-  r.rDR = -r.c.invdR;
-  r.r3G = 1.0 / (3.0 * r.c.G);
+  r.df = r.f * (1.0 + 4.0 * r.nu) * rden;
+  VMConst& c = r.c;
+  c.Ei = Iso{r.f * (1.0 - r.nu), r.f * r.nu, 0.5 * r.E * r.r1nu};
+  c.G = c.Ei.c44;
+  c.fy0 = vonMises ? props[2] : 0.0;
+  c.H = vonMises ? props[3] : 0.0;
+  c.dfy = vonMises ? props[4] : 0.0;
+  c.delta = vonMises ? props[5] : 0.0;
+  const double g3 = 3.0 * c.G, q = 1.0 / (g3 + c.H);
+  c.tfac = g3 * q;
+  r.rDR = sqrt(1.5) * q;
+  c.invdR = -r.rDR;
+  c.sq6G = sqrt(6.0) * c.G;
+  c.g15 = 2.0 * sqrt(1.5) * c.G;
+  r.r3G = (2.0 / 3.0) * n1 * r.rE;
   return r;
 }
 
@@ -267,16 +286,15 @@ __device__ inline void linear_elastic_plane_stress_reverse(double E, double nu, 
              rBar / ((1.0 - nu) * (1.0 - nu));
 }
 
-// Coordinate adjoint of one point (see the head comment), accumulated into a.gX.  u and pb: the
-// element's dU and PBar as staged by phase 0 (float-float relative to node 0 in the FF form, which
-// leaves M unchanged: sum_a G_a = 0).
-template <int SHAPE, int RULE, bool FF>
-__device__ __forceinline__ void coordinate_adjoint(const SSAdjointArgs& a, int64_t e, int q, int64_t pt, int64_t stride,
-                                                   double s, const VMConst& mc, bool vm, bool planeStress,
-                                                   const double sig0[6], double k0, const double de[6],
-                                                   const double deBar[6], const double bp[6], const double* u,
-                                                   const double* pb) {
-  constexpr int DIM = ShapeInfo<SHAPE>::DIM, NN = ShapeInfo<SHAPE>::NN;
+// Coordinate adjoint of one point (see the head comment): gX[n][c] += sum_k Q[k][c] dN_n/dX_k + r_n W[c], with Hu and
+// Hp the gradients of dU and PBar and M = deBar Hu - s sigma Hp; W (Hexa20) feeds the quirk row of J.
+template <int SHAPE, int RULE, int DIM>
+__device__ __forceinline__ void coordinate_adjoint(const SSAdjointArgs& a, int64_t e, int q, double s, const VMConst& mc,
+                                                   bool vm, bool planeStress, const double sig0[6], double k0,
+                                                   const double de[6], const double deBar[6], const double bp[6],
+                                                   const double Hu[DIM][DIM], const double Hp[DIM][DIM],
+                                                   double Q[DIM][DIM], double W[3]) {
+  constexpr int NN = ShapeInfo<SHAPE>::NN;
   // the new stress (the FP64 form of the forward update)
   double sn[6], kn = k0, dp[6];
   for (int f = 0; f < 6; ++f) {
@@ -306,34 +324,25 @@ __device__ __forceinline__ void coordinate_adjoint(const SSAdjointArgs& a, int64
   } else {
     sBar = -(sn[0] * bp[0] + sn[1] * bp[1] + sn[3] * bp[3]);
   }
-  auto val = [&](const double* arr, int k) {
-    if constexpr (FF)
-      return ff_to_double(reinterpret_cast<const ff*>(arr)[k]);
-    else
-      return arr[k];
-  };
-  double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  for (int n = 0; n < NN; ++n) {
-    double G[3], ua[3], pa[3], Gb[3];
+  double M[DIM][DIM];
+#pragma unroll
+  for (int k = 0; k < DIM; ++k)
+#pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      G[c] = a.geomG[(int64_t)(c * NN + n) * stride + pt];
-      ua[c] = val(u, n * DIM + c);
-      pa[c] = val(pb, n * DIM + c);
+      double v = 0.0, w = 0.0;
+#pragma unroll
+      for (int l = 0; l < DIM; ++l) {
+        v = fma(Db[k][l], Hu[l][c], v);
+        w = fma(S[k][l], Hp[l][c], w);
+      }
+      M[k][c] = fma(-s, w, v);
+      Q[k][c] = (k == c ? s * sBar : 0.0) - M[k][c];
     }
-    for (int k = 0; k < DIM; ++k) {
-      double v = 0.0;
-      for (int l = 0; l < DIM; ++l) v += Db[k][l] * ua[l] - s * S[k][l] * pa[l];
-      Gb[k] = v;
-    }
-    for (int k = 0; k < DIM; ++k)
-      for (int c = 0; c < DIM; ++c) M[k][c] += Gb[k] * G[c];
-  }
   // the Hexa20 quirk row of J (J[2][c] += (zeta - xi) sum_a r_a X_a[c]): Jbar[2][c] feeds it
-  double Jb2[3] = {0, 0, 0}, qk = 0.0;
   if constexpr (SHAPE == EFE_HEXA20) {
     double xi, eta, zeta, w;
     quadrature_point(RULE, q, xi, eta, zeta, w);
-    qk = zeta - xi;
+    const double qk = zeta - xi;
     const double p[3] = {eta, xi, zeta};
     double D[3][NN];
     shape_derivatives<SHAPE>(p, D);
@@ -350,26 +359,17 @@ __device__ __forceinline__ void coordinate_adjoint(const SSAdjointArgs& a, int64
     for (int c = 0; c < 3; ++c) {
       double v = s * sBar * iJ[c][2];
       for (int k = 0; k < 3; ++k) v -= iJ[k][2] * M[k][c];
-      Jb2[c] = v;
-    }
-  }
-  for (int n = 0; n < NN; ++n) {
-    const int32_t node = a.conn[e * NN + n];
-    for (int c = 0; c < DIM; ++c) {
-      double v = s * sBar * a.geomG[(int64_t)(c * NN + n) * stride + pt];
-      for (int k = 0; k < DIM; ++k) v -= M[k][c] * a.geomG[(int64_t)(k * NN + n) * stride + pt];
-      if constexpr (SHAPE == EFE_HEXA20) v += qk * a.fix.r[n] * Jb2[c];
-      atomicAdd(a.gX + (int64_t)node * DIM + c, v);
+      W[c] = qk * v;
     }
   }
 }
 
-template <int SHAPE, int RULE>
+template <int SHAPE, int RULE, bool GX>
 struct SSAdjointTile {
   static constexpr int DIM = ShapeInfo<SHAPE>::DIM, NN = ShapeInfo<SHAPE>::NN, NQ = RuleInfo<RULE>::NQ;
   static constexpr int NDOF = NN * DIM, NT = 128;
-  // per element: dU_e and PBar_e; its points' dN/dX (NDOF x NQ, 8 bytes each: doubles, or float-float
-  // hi and lo floats), property adjoints (6) and strain adjoints (6)
+  // per element: dU_e and PBar_e; its points' dN/dX (NDOF x NQ, 8 bytes each: doubles, then digits), property adjoints
+  // (6) and strain adjoints (6)
   static constexpr size_t per_el = sizeof(double) * (2 * NDOF + NQ * NDOF + NQ * 12);
   static constexpr int EPB0 = NT / NQ > 0 ? NT / NQ : 1;
   static constexpr int EPB = (size_t)EPB0 * per_el <= 96 * 1024 ? EPB0 : (int)((96 * 1024) / per_el);
@@ -377,177 +377,180 @@ struct SSAdjointTile {
   // the staged dN/dX: row r = l NN + a (component l of dN_a/dX) over the tile's points, an odd row
   // stride so that the per-DOF reads of phase C (different rows, one point) spread over the banks
   static constexpr int NP = EPB * NQ, NPS = NP | 1;
+  // dU and PBar; in their place, for the coordinate adjoint, fx [NP][DIM][DIM]: Q
+  static constexpr size_t up_bytes = sizeof(double) * 2 * EPB * NDOF, qq_bytes = GX ? sizeof(double) * NP * DIM * DIM : 0;
   static constexpr size_t u_off = 0, p_off = u_off + sizeof(double) * EPB * NDOF,
-                          g_off = p_off + sizeof(double) * EPB * NDOF,
+                          g_off = up_bytes > qq_bytes ? up_bytes : qq_bytes,
                           q_off = g_off + sizeof(double) * NDOF * NPS,  // double [NP][6]: property adjoints
-                          d_off = q_off + sizeof(double) * NP * 6,      // double or ff [NP][6]: strain adjoints
+                          d_off = q_off + sizeof(double) * NP * 6,      // fx [NP][6]: strain adjoints
                           c_off = d_off + sizeof(double) * NP * 6,      // SSRevConst [EPB]
-                          bytes = c_off + sizeof(SSRevConst) * EPB;
+                          w_off = c_off + sizeof(SSRevConst) * EPB,     // double [NP][3]: W
+                          e_off = w_off + (GX && SHAPE == EFE_HEXA20 ? sizeof(double) * NP * 3 : 0),
+                          bytes = e_off + sizeof(int) * 4 * EPB;  // int [EPB][4]: scales of dU, PBar, B^T deBar, Q
+  static_assert(NP <= NT, "a thread per point");
+  static_assert(2 * ((NN + 1) / 2) <= 31 && NQ <= 31, "products of a fixed-point sum");
 };
 
-// FF: the three B-products (B dU, B PBar, B^T deBar) in float-float arithmetic on the FP32 pipe from the
-// float-float geometry (geomG32 + geomGlo), with nodal values taken relative to the element's first
-// node (sum_a dN_a/dX = 0); the reverse return map stays FP64.  ~2^-48 relative accuracy.
-// Phase 0 stages the tile's dN/dX rows in shared memory (cp.async), so that phase A (one thread per
-// point: B dU, B PBar, the reverse update) and phase C (one thread per element DOF: B^T deBar summed
-// over the points) read it there rather than twice from global memory.
-template <int SHAPE, int RULE, bool FF, bool GX>
-__global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE>::NT) adjoint_ss_kernel(SSAdjointArgs a) {
-  using T = SSAdjointTile<SHAPE, RULE>;
+// The three B-products (B dU, B PBar, B^T deBar) run in fixed-point integers (efe_fixed.cuh) on digits of dN/dX, of the
+// nodal values, taken relative to the element's first node (sum_a dN_a/dX = 0), and of deBar; the FP64 pipe is left with the
+// reverse return map.
+// Phase 0 stages the tile's dN/dX rows in shared memory (cp.async), where each point's thread converts its column, so that
+// phase A (one thread per point: B dU, B PBar, the reverse update) and phase C (one thread per element DOF: B^T deBar
+// summed over the points) read it there rather than twice from global memory.
+template <int SHAPE, int RULE, bool GX>
+__global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss_kernel(SSAdjointArgs a) {
+  using T = SSAdjointTile<SHAPE, RULE, GX>;
   constexpr int DIM = T::DIM, NN = T::NN, NQ = T::NQ, NDOF = T::NDOF, EPB = T::EPB, NT = T::NT, NPS = T::NPS;
   extern __shared__ __align__(128) unsigned char smem[];
-  double* su = reinterpret_cast<double*>(smem + T::u_off);
-  double* sp = reinterpret_cast<double*>(smem + T::p_off);
-  float* sGh = reinterpret_cast<float*>(smem + T::g_off);  // FF: hi floats, then lo floats
-  float* sGl = sGh + NDOF * NPS;
-  double* sGd = reinterpret_cast<double*>(smem + T::g_off);  // FP64 dN/dX
+  fx* su = reinterpret_cast<fx*>(smem + T::u_off);
+  fx* sp = reinterpret_cast<fx*>(smem + T::p_off);
+  double* sud = reinterpret_cast<double*>(smem + T::u_off);  // dU, then PBar of all elements
+  double* sGd = reinterpret_cast<double*>(smem + T::g_off);
+  fx* sG = reinterpret_cast<fx*>(smem + T::g_off);
   double* sg = reinterpret_cast<double*>(smem + T::q_off);
-  double* sd = reinterpret_cast<double*>(smem + T::d_off);
+  fx* sd = reinterpret_cast<fx*>(smem + T::d_off);
+  fx* sQ = reinterpret_cast<fx*>(smem + T::u_off);
+  double* sW = reinterpret_cast<double*>(smem + T::w_off);
   SSRevConst* src = reinterpret_cast<SSRevConst*>(smem + T::c_off);
+  int* sem = reinterpret_cast<int*>(smem + T::e_off);
   const int64_t e0 = (int64_t)blockIdx.x * EPB;
   const int64_t nEl = a.nEl, stride = nEl * NQ;
   const bool vm = a.material == EFE_MAT_VON_MISES;
   const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB;  // elements of this tile
 
-  // ---- phase 0: dN/dX rows (cp.async), dU_e and PBar_e, the elements' constants
-  for (int t = threadIdx.x; t < NDOF * nLoc * NQ; t += NT) {
-    const int r = t / (nLoc * NQ), j = t - r * (nLoc * NQ);
-    const int64_t gi = (int64_t)r * stride + e0 * NQ + j;
-    if constexpr (FF) {
-      tc::cp_async4(sGh + r * NPS + j, a.geomG32 + gi);
-      tc::cp_async4(sGl + r * NPS + j, a.geomGlo + gi);
-    } else {
-      tc::cp_async8(sGd + r * NPS + j, a.geomG + gi);
-    }
+  // ---- phase 0: dN/dX of the thread's point (cp.async), dU_e and PBar_e, the elements' constants
+  const int pl = threadIdx.x;  // the point in the tile
+  const bool live = pl < nLoc * NQ;
+  if (live) {
+    const double* gp = a.geomG + e0 * NQ + pl;
+#pragma unroll 10
+    for (int r = 0; r < NDOF; ++r) tc::cp_async8(sGd + r * NPS + pl, gp + (int64_t)r * stride);
   }
-  if (threadIdx.x < nLoc) src[threadIdx.x] = ss_rev_const(a.props + (e0 + threadIdx.x) * a.nProps, vm);
-  for (int t = threadIdx.x; t < EPB * NN; t += NT) {
-    const int le = t / NN, n = t % NN;
-    const int64_t e = e0 + le;
-    if (e >= nEl) continue;
-    const int32_t dof = a.nodeDof[a.conn[e * NN + n]];
-    if constexpr (FF) {
-      const int32_t dof0 = a.nodeDof[a.conn[e * NN]];
-      ff* uf = reinterpret_cast<ff*>(su);
-      ff* pf = reinterpret_cast<ff*>(sp);
-      for (int c = 0; c < DIM; ++c) {
-        uf[le * NDOF + n * DIM + c] = ff_split(a.dU[dof + c] - a.dU[dof0 + c]);
-        pf[le * NDOF + n * DIM + c] = ff_split(a.Pbar ? a.Pbar[dof + c] - a.Pbar[dof0 + c] : 0.0);
-      }
-    } else {
-      for (int c = 0; c < DIM; ++c) {
-        su[le * NDOF + n * DIM + c] = a.dU[dof + c];
-        sp[le * NDOF + n * DIM + c] = a.Pbar ? a.Pbar[dof + c] : 0.0;
-      }
+  for (int t = threadIdx.x; t < 4 * EPB; t += NT) sem[t] = 0;
+  __syncthreads();
+  if (NT - 1 - (int)threadIdx.x < nLoc) {
+    const int le = NT - 1 - threadIdx.x;
+    src[le] = ss_rev_const(a.props + (e0 + le) * a.nProps, vm);
+  }
+  for (int t = threadIdx.x; t < nLoc * NN; t += NT) {
+    const int le = t / NN, n = t - le * NN;
+    const int32_t* en = a.conn + (e0 + le) * NN;
+    const int32_t dof = a.nodeDof[en[n]], dof0 = a.nodeDof[en[0]];
+    int eu = 0, ep = 0;
+    for (int c = 0; c < DIM; ++c) {
+      const double u = a.dU[dof + c] - a.dU[dof0 + c], p = a.Pbar ? a.Pbar[dof + c] - a.Pbar[dof0 + c] : 0.0;
+      sud[le * NDOF + n * DIM + c] = u;
+      sud[EPB * NDOF + le * NDOF + n * DIM + c] = p;
+      eu = fx_max_exponent(eu, u);
+      ep = fx_max_exponent(ep, p);
     }
+    atomicMax(sem + le * 4, eu);
+    atomicMax(sem + le * 4 + 1, ep);
   }
   tc::cp_async_wait_all();
   __syncthreads();
+  for (int t = threadIdx.x; t < 2 * nLoc * NDOF; t += NT) {
+    const int w = t >= nLoc * NDOF, k = t - w * nLoc * NDOF;
+    su[w * EPB * NDOF + k] = fx_make(sud[w * EPB * NDOF + k], sem[k / NDOF * 4 + w]);
+  }
+  int eg = 0;
+  if (live) {
+#pragma unroll 10
+    for (int r = 0; r < NDOF; ++r) eg = fx_max_exponent(eg, sGd[r * NPS + pl]);
+#pragma unroll 4
+    for (int r = 0; r < NDOF; ++r) sG[r * NPS + pl] = fx_make(sGd[r * NPS + pl], eg);
+  }
+  __syncthreads();
 
   // ---- phase A: one thread per point
-  for (int t = threadIdx.x; t < EPB * NQ; t += NT) {
-    const int le = t / NQ, q = t % NQ;
-    const int64_t e = e0 + le;
-    if (e >= nEl) continue;
-    const int64_t pt = e * NQ + q;
-    const int pl = le * NQ + q;  // the point in the tile
+  double deBar[6], Q[DIM][DIM];
+  if (live) {
+    const int le = pl / NQ, q = pl - le * NQ;
+    const int64_t e = e0 + le, pt = e0 * NQ + pl;
     const double s = a.geomS[pt];
     // B u and B PBar (small-strain Voigt 11,22,33,12,13,23, engineering shear)
-    double de[6] = {0, 0, 0, 0, 0, 0}, bp[6] = {0, 0, 0, 0, 0, 0};
-    if constexpr (FF) {
-      const ff* uf = reinterpret_cast<const ff*>(su) + le * NDOF;
-      const ff* pf = reinterpret_cast<const ff*>(sp) + le * NDOF;
-      ff ad[6] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}}, ab[6] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
+    // at most 20 products to a sum: half of the nodes at a time beyond eight
+    constexpr int PARTS = NN > 8 ? 2 : 1;
+    auto strain = [&](const fx* v, int em, double out[6]) {
+      int64_t sum[6] = {0, 0, 0, 0, 0, 0};
+      for (int part = 0; part < PARTS; ++part) {
+        FxSum f[6] = {};
+#pragma unroll 2
+        for (int n = part * (NN / PARTS); n < (part + 1) * (NN / PARTS); ++n) {
+          const fx gx = sG[n * NPS + pl], gy = sG[(NN + n) * NPS + pl];
+          const fx vx = v[n * DIM], vy = v[n * DIM + 1];
+          fx_fma(f[0], gx, vx);
+          fx_fma(f[1], gy, vy);
+          fx_fma(f[3], gy, vx);
+          fx_fma(f[3], gx, vy);
+          if constexpr (DIM == 3) {
+            const fx gz = sG[(2 * NN + n) * NPS + pl], vz = v[n * DIM + 2];
+            fx_fma(f[2], gz, vz);
+            fx_fma(f[4], gz, vx);
+            fx_fma(f[4], gx, vz);
+            fx_fma(f[5], gz, vy);
+            fx_fma(f[5], gy, vz);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) sum[k] += fx_int(f[k], 1 - PARTS);
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) out[k] = fx_value(sum[k], em + eg + PARTS - 1);
+    };
+    // the gradient as well: out from its symmetric part, summed in integers
+    auto gradient = [&](const fx* v, int em, double out[6], double H[DIM][DIM]) {
+      FxSum f[DIM][DIM] = {};
+#pragma unroll 2
       for (int n = 0; n < NN; ++n) {
-        const ff gx = ff{sGh[n * NPS + pl], sGl[n * NPS + pl]};
-        const ff gy = ff{sGh[(NN + n) * NPS + pl], sGl[(NN + n) * NPS + pl]};
-        if constexpr (DIM == 3) {
-          const ff gz = ff{sGh[(2 * NN + n) * NPS + pl], sGl[(2 * NN + n) * NPS + pl]};
-          const ff ux = uf[n * 3], uy = uf[n * 3 + 1], uz = uf[n * 3 + 2];
-          const ff px = pf[n * 3], py = pf[n * 3 + 1], pz = pf[n * 3 + 2];
-          ff_fma(ad[0], gx, ux);
-          ff_fma(ad[1], gy, uy);
-          ff_fma(ad[2], gz, uz);
-          ff_fma(ad[3], gy, ux);
-          ff_fma(ad[3], gx, uy);
-          ff_fma(ad[4], gz, ux);
-          ff_fma(ad[4], gx, uz);
-          ff_fma(ad[5], gz, uy);
-          ff_fma(ad[5], gy, uz);
-          ff_fma(ab[0], gx, px);
-          ff_fma(ab[1], gy, py);
-          ff_fma(ab[2], gz, pz);
-          ff_fma(ab[3], gy, px);
-          ff_fma(ab[3], gx, py);
-          ff_fma(ab[4], gz, px);
-          ff_fma(ab[4], gx, pz);
-          ff_fma(ab[5], gz, py);
-          ff_fma(ab[5], gy, pz);
-        } else {
-          const ff ux = uf[n * 2], uy = uf[n * 2 + 1];
-          const ff px = pf[n * 2], py = pf[n * 2 + 1];
-          ff_fma(ad[0], gx, ux);
-          ff_fma(ad[1], gy, uy);
-          ff_fma(ad[3], gy, ux);
-          ff_fma(ad[3], gx, uy);
-          ff_fma(ab[0], gx, px);
-          ff_fma(ab[1], gy, py);
-          ff_fma(ab[3], gy, px);
-          ff_fma(ab[3], gx, py);
+        fx g[DIM];
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) g[c] = sG[(c * NN + n) * NPS + pl];
+#pragma unroll
+        for (int l = 0; l < DIM; ++l) {
+          const fx x = v[n * DIM + l];
+#pragma unroll
+          for (int c = 0; c < DIM; ++c) fx_fma(f[l][c], x, g[c]);
         }
       }
-      for (int f = 0; f < 6; ++f) {
-        de[f] = ff_to_double(ad[f]);
-        bp[f] = ff_to_double(ab[f]);
-      }
-    } else {
-      const double* u = su + le * NDOF;
-      const double* pb = sp + le * NDOF;
-      for (int n = 0; n < NN; ++n) {
-        const double gx = sGd[n * NPS + pl], gy = sGd[(NN + n) * NPS + pl];
-        if constexpr (DIM == 3) {
-          const double gz = sGd[(2 * NN + n) * NPS + pl];
-          const double ux = u[n * 3], uy = u[n * 3 + 1], uz = u[n * 3 + 2];
-          const double px = pb[n * 3], py = pb[n * 3 + 1], pz = pb[n * 3 + 2];
-          de[0] = fma(gx, ux, de[0]);
-          de[1] = fma(gy, uy, de[1]);
-          de[2] = fma(gz, uz, de[2]);
-          de[3] = fma(gx, uy, fma(gy, ux, de[3]));
-          de[4] = fma(gx, uz, fma(gz, ux, de[4]));
-          de[5] = fma(gy, uz, fma(gz, uy, de[5]));
-          bp[0] += gx * px;
-          bp[1] += gy * py;
-          bp[2] += gz * pz;
-          bp[3] += gy * px + gx * py;
-          bp[4] += gz * px + gx * pz;
-          bp[5] += gz * py + gy * pz;
-        } else {
-          const double ux = u[n * 2], uy = u[n * 2 + 1];
-          const double px = pb[n * 2], py = pb[n * 2 + 1];
-          de[0] += gx * ux;
-          de[1] += gy * uy;
-          de[3] += gy * ux + gx * uy;
-          bp[0] += gx * px;
-          bp[1] += gy * py;
-          bp[3] += gy * px + gx * py;
+      int64_t I[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+      for (int l = 0; l < DIM; ++l)
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+          I[l][c] = fx_int(f[l][c], -1);
+          H[l][c] = fx_value(I[l][c], em + eg + 1);
         }
-      }
-    }
-    // seeds: the new state's adjoint, plus P_e = -sum_q s B^T sig  =>  sigBar -= s B PBar
-    double sBar[6], eBar[6], kBar = 0.0;
+      const int64_t sum[6] = {I[0][0], I[1][1], I[2][2], I[0][1] + I[1][0], I[0][2] + I[2][0], I[1][2] + I[2][1]};
+#pragma unroll
+      for (int k = 0; k < 6; ++k) out[k] = fx_value(sum[k], em + eg + 1);
+    };
+    // seeds and the state before the increment, loaded ahead of the sums
+    double sBar[6], eBar[6], kBar = 0.0, sig0[6], k0 = 0.0;
+#pragma unroll
     for (int f = 0; f < 6; ++f) {
-      sBar[f] = (a.barIn ? a.barIn[(int64_t)f * stride + pt] : 0.0) - s * bp[f];
+      sBar[f] = a.barIn ? a.barIn[(int64_t)f * stride + pt] : 0.0;
       eBar[f] = a.barIn ? a.barIn[(int64_t)(6 + f) * stride + pt] : 0.0;
+      sig0[f] = a.stateBefore[(int64_t)f * stride + pt];
     }
     if (vm && a.barIn) kBar = a.barIn[(int64_t)12 * stride + pt];
-    double sig0[6], k0 = 0.0;
-    for (int f = 0; f < 6; ++f) sig0[f] = a.stateBefore[(int64_t)f * stride + pt];
     if (vm) k0 = a.stateBefore[(int64_t)12 * stride + pt];
+    double de[6], bp[6];
+    double Hu[DIM][DIM], Hp[DIM][DIM];
+    if constexpr (GX) {
+      gradient(su + le * NDOF, sem[le * 4], de, Hu);
+      gradient(sp + le * NDOF, sem[le * 4 + 1], bp, Hp);
+    } else {
+      strain(su + le * NDOF, sem[le * 4], de);
+      strain(sp + le * NDOF, sem[le * 4 + 1], bp);
+    }
+    // P_e = -sum_q s B^T sig  =>  sigBar -= s B PBar
+#pragma unroll
+    for (int f = 0; f < 6; ++f) sBar[f] -= s * bp[f];
     const double* props = a.props + e * a.nProps;
     const SSRevConst& rc = src[le];
     const VMConst& mc = rc.c;
     double sig0Bar[6] = {0, 0, 0, 0, 0, 0}, k0Bar = 0.0, pBar[6] = {0, 0, 0, 0, 0, 0};
-    double deBar[6];
     for (int f = 0; f < 6; ++f) deBar[f] = eBar[f];  // eps = eps0 + de
     bool planeStress = false;
     if constexpr (DIM == 2) planeStress = a.planeStress;
@@ -563,57 +566,82 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE>::NT) adjoint_ss_ker
       hypo3d_reverse(rc, vm, sig0, k0, de, sBar, kBar, sig0Bar, k0Bar, deBar, pBar);
     }
     if (a.barOut) {
+      // all loads before the first store, which they could not pass
+#pragma unroll
       for (int f = 0; f < 6; ++f) {
-        a.barOut[(int64_t)f * stride + pt] += sig0Bar[f];
-        a.barOut[(int64_t)(6 + f) * stride + pt] += eBar[f];
+        sig0Bar[f] += a.barOut[(int64_t)f * stride + pt];
+        eBar[f] += a.barOut[(int64_t)(6 + f) * stride + pt];
       }
-      if (vm) a.barOut[(int64_t)12 * stride + pt] += k0Bar;
+      if (vm) k0Bar += a.barOut[(int64_t)12 * stride + pt];
+#pragma unroll
+      for (int f = 0; f < 6; ++f) {
+        a.barOut[(int64_t)f * stride + pt] = sig0Bar[f];
+        a.barOut[(int64_t)(6 + f) * stride + pt] = eBar[f];
+      }
+      if (vm) a.barOut[(int64_t)12 * stride + pt] = k0Bar;
     }
     double* gq = sg + pl * 6;
     for (int k = 0; k < 6; ++k) gq[k] = pBar[k];
-    if constexpr (GX) coordinate_adjoint<SHAPE, RULE, FF>(a, e, q, pt, stride, s, mc, vm, planeStress, sig0, k0, de,
-                                                 deBar, bp, su + le * NDOF, sp + le * NDOF);
-    // the strain adjoint, for B^T deBar in phase C
-    if constexpr (FF) {
-      ff* df = reinterpret_cast<ff*>(sd) + pl * 6;
-      for (int f = 0; f < 6; ++f) df[f] = ff_split(deBar[f]);
-    } else {
-      for (int f = 0; f < 6; ++f) sd[pl * 6 + f] = deBar[f];
+    if constexpr (GX) {
+      double W[3] = {0.0, 0.0, 0.0};
+      coordinate_adjoint<SHAPE, RULE, DIM>(a, e, q, s, mc, vm, planeStress, sig0, k0, de, deBar, bp, Hu, Hp, Q, W);
+      int eq = 0;
+#pragma unroll
+      for (int k = 0; k < DIM; ++k)
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) eq = fx_max_exponent(eq, Q[k][c]);
+      atomicMax(sem + le * 4 + 3, eq + eg);
+      if constexpr (SHAPE == EFE_HEXA20)
+        for (int c = 0; c < 3; ++c) sW[pl * 3 + c] = W[c];
     }
+    int ed = 0;
+    for (int f = 0; f < 6; ++f) ed = fx_max_exponent(ed, deBar[f]);
+    atomicMax(sem + le * 4 + 2, ed + eg);
+  }
+  __syncthreads();
+  if (live) {
+    for (int f = 0; f < 6; ++f) sd[pl * 6 + f] = fx_make(deBar[f], sem[pl / NQ * 4 + 2] - eg);
+    if constexpr (GX)
+      for (int k = 0; k < DIM; ++k)
+        for (int c = 0; c < DIM; ++c) sQ[(pl * DIM + k) * DIM + c] = fx_make(Q[k][c], sem[pl / NQ * 4 + 3] - eg);
   }
   __syncthreads();
 
   // ---- phase C: per element DOF (node n, component c): sum over the points of (B^T deBar)_(n,c) =
   // row c of the symmetric strain adjoint (Voigt, engineering shear) times dN_n/dX; one atomic per
   // element DOF.  Per element property: plain stores (one thread owns an element's property).
-  for (int t = threadIdx.x; t < EPB * NDOF; t += NT) {
-    const int le = t / NDOF, k = t % NDOF, n = k / DIM, c = k % DIM;
+  for (int t = threadIdx.x; t < nLoc * NDOF; t += NT) {
+    const int le = t / NDOF, k = t - le * NDOF, n = k / DIM, c = k - n * DIM;
     const int64_t e = e0 + le;
-    if (e >= nEl) continue;
     // row c: 3D (11 12 13 | 12 22 23 | 13 23 33) = Voigt (0 3 4 | 3 1 5 | 4 5 2); 2D (0 3 | 3 1)
     const int v0 = c == 0 ? 0 : (c == 1 ? 3 : 4), v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
-    double v;
-    if constexpr (FF) {
-      const ff* df = reinterpret_cast<const ff*>(sd);
-      ff acc{0, 0};
-      for (int q = 0; q < NQ; ++q) {
-        const int pl = le * NQ + q;
-        ff_fma(acc, df[pl * 6 + v0], ff{sGh[n * NPS + pl], sGl[n * NPS + pl]});
-        ff_fma(acc, df[pl * 6 + v1], ff{sGh[(NN + n) * NPS + pl], sGl[(NN + n) * NPS + pl]});
-        if constexpr (DIM == 3) ff_fma(acc, df[pl * 6 + v2], ff{sGh[(2 * NN + n) * NPS + pl], sGl[(2 * NN + n) * NPS + pl]});
-      }
-      v = ff_to_double(acc);
-    } else {
-      v = 0.0;
-      for (int q = 0; q < NQ; ++q) {
-        const int pl = le * NQ + q;
-        double r = sd[pl * 6 + v0] * sGd[n * NPS + pl] + sd[pl * 6 + v1] * sGd[(NN + n) * NPS + pl];
-        if constexpr (DIM == 3) r += sd[pl * 6 + v2] * sGd[(2 * NN + n) * NPS + pl];
-        v += r;
-      }
+    FxSum f[3] = {};  // one for each direction
+#pragma unroll 3
+    for (int q = 0; q < NQ; ++q) {
+      const int p = le * NQ + q;
+      fx_fma(f[0], sd[p * 6 + v0], sG[n * NPS + p]);
+      fx_fma(f[1], sd[p * 6 + v1], sG[(NN + n) * NPS + p]);
+      if constexpr (DIM == 3) fx_fma(f[2], sd[p * 6 + v2], sG[(2 * NN + n) * NPS + p]);
     }
-    const int32_t dof = a.nodeDof[a.conn[e * NN + n]] + c;
-    atomicAdd(a.dUbar + dof, v);
+    const double v = fx_value(fx_int(f[0], -2) + fx_int(f[1], -2) + fx_int(f[2], -2), sem[le * 4 + 2] + 2);
+    const int32_t node = a.conn[e * NN + n];
+    atomicAdd(a.dUbar + a.nodeDof[node] + c, v);
+    if constexpr (GX) {
+      FxSum h[3] = {};
+#pragma unroll 3
+      for (int q = 0; q < NQ; ++q) {
+        const int p = le * NQ + q;
+#pragma unroll
+        for (int l = 0; l < DIM; ++l) fx_fma(h[l], sQ[(p * DIM + l) * DIM + c], sG[(l * NN + n) * NPS + p]);
+      }
+      double x = fx_value(fx_int(h[0], -2) + fx_int(h[1], -2) + fx_int(h[2], -2), sem[le * 4 + 3] + 2);
+      if constexpr (SHAPE == EFE_HEXA20) {
+        double w = 0.0;
+        for (int q = 0; q < NQ; ++q) w += sW[(le * NQ + q) * 3 + c];
+        x = fma(a.fix.r[n], w, x);
+      }
+      atomicAdd(a.gX + (int64_t)node * DIM + c, x);
+    }
   }
   if (a.gProps) {
     const int np = a.nProps < 6 ? a.nProps : 6;
@@ -630,15 +658,14 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE>::NT) adjoint_ss_ker
 
 template <int SHAPE, int RULE>
 cudaError_t launch_adjoint_ss(const SSAdjointArgs& a, cudaStream_t st) {
-  using T = SSAdjointTile<SHAPE, RULE>;
+  using T = SSAdjointTile<SHAPE, RULE, true>;  // EPB and NT are those of the pass without gX
   if (a.nEl == 0) return cudaSuccess;
-  const bool ff = a.geomG32 && a.geomGlo;
-  auto kern = a.gX ? (ff ? adjoint_ss_kernel<SHAPE, RULE, true, true> : adjoint_ss_kernel<SHAPE, RULE, false, true>)
-                   : (ff ? adjoint_ss_kernel<SHAPE, RULE, true, false> : adjoint_ss_kernel<SHAPE, RULE, false, false>);
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::bytes);
+  auto kern = a.gX ? adjoint_ss_kernel<SHAPE, RULE, true> : adjoint_ss_kernel<SHAPE, RULE, false>;
+  const size_t bytes = a.gX ? T::bytes : SSAdjointTile<SHAPE, RULE, false>::bytes;
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   const int64_t blocks = (a.nEl + T::EPB - 1) / T::EPB;
-  kern<<<(unsigned)blocks, T::NT, T::bytes, st>>>(a);
+  kern<<<(unsigned)blocks, T::NT, bytes, st>>>(a);
   return cudaGetLastError();
 }
 
