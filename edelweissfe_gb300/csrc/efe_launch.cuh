@@ -10,20 +10,21 @@ namespace efe {
 // thread in phase A), 128 threads, at most 72 KB of shared memory so that three CTAs share an SM.
 // Variant 1: about 256 points and 256 threads per CTA, up to 110 KB (one or two CTAs per SM).
 // The autotuner (edelweissfe_gb300/autotune.py) picks one per group by timing both.
+constexpr int SMALL_TILE = 4;
 template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT>
 struct TileOf {
   // variant 0: 128 threads, ~128 points, 3 CTAs/SM where they fit; 1: 256 threads, ~256 points;
   // 2: variant 0's tile with 4 CTAs/SM where shared memory allows (the compiler then holds the
-  // kernel to 128 registers per thread)
+  // kernel to 128 registers per thread); SMALL_TILE: about 16 points, for groups that fill few SMs
   static constexpr int NQ = RuleInfo<RULE>::NQ;
   static constexpr size_t per_element = LayoutOf<SHAPE, RULE, FORM, KT, 1>::bytes;
   static constexpr size_t budget = VARIANT == 1 ? 110 * 1024 : 72 * 1024;
-  static constexpr int points = VARIANT == 1 ? 256 : 128;
+  static constexpr int points = VARIANT == 1 ? 256 : VARIANT == SMALL_TILE ? 16 : 128;
   static constexpr int fit = (int)(budget / per_element);
   static constexpr int want = (points + NQ - 1) / NQ;
   static constexpr int e0 = fit < want ? fit : want;
   static constexpr int EPB = e0 < 1 ? 1 : (e0 > 32 ? 32 : e0);
-  static constexpr int NT = VARIANT == 1 ? 256 : 128;
+  static constexpr int NT = VARIANT == 1 ? 256 : VARIANT == SMALL_TILE && ShapeInfo<SHAPE>::NN <= 8 ? 64 : 128;
   static constexpr size_t bytes = LayoutOf<SHAPE, RULE, FORM, KT, EPB>::bytes;
   static constexpr int MINB = VARIANT == 1 ? 1
                               : (VARIANT == 2 && bytes <= 56 * 1024) ? 4
@@ -32,8 +33,9 @@ struct TileOf {
 // The warp tile of small-strain Hexa8 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: six CTAs of
 // four warps per SM hold the kernel to 80 registers (40 B of spills); five CTAs (96 registers) or four (128) run in 1.01
 // and 1.06 times its time on 262144 elements, 1.00 and 1.05 times on 65231.
+template <int VARIANT>
 struct WarpTile {
-  static constexpr int NT = 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = 6;
+  static constexpr int NT = VARIANT == SMALL_TILE ? 32 : 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = VARIANT == SMALL_TILE ? 1 : 6;
   static constexpr size_t bytes = SS3Hexa8Layout<NT>::bytes;
 };
 // The two-element tile of small-strain Hexa20 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: five CTAs per
@@ -43,7 +45,7 @@ struct Hexa20Tile {
   static constexpr size_t bytes = SS3Hexa20Layout::bytes;
 };
 template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT = 0>
-struct Tile : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile,
+struct Tile : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile<VARIANT>,
                                typename std::conditional<FORM == SS3 && ss3_hexa20_tile<SHAPE, RULE, KT>(), Hexa20Tile,
                                                          TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type>::type {};
 
@@ -123,6 +125,19 @@ cudaError_t launch_assemble(const GroupArgs& g, cudaStream_t st) {
   constexpr bool ffTile = FF && FORM != SS3;  // the small-strain solids form their B-products in integers in either mode
   if constexpr (has_tc_variant<SHAPE, RULE, FORM, KT>()) {
     if (g.tileVariant == 3) return launch_assemble_tc<FF>(g, st);
+  }
+  // A small group's ordinary tiles leave most SMs without one, and a tile's phases one after the other are then the
+  // whole time: small tiles up to two per SM.  320 CPE4 elements (fp64) 11 us against 19, 1200 CPE8R 20 against 45, 512
+  // C3D8TL (mixed) 15 against 19, 1000 C3D8 (mixed) 18.4 against 19.5; beyond, 1000 C3D8 (fp64) 32 against 28 and 4000 CPE4
+  // 35 against 22.
+  using Small = Tile<SHAPE, RULE, FORM, KT, SMALL_TILE>;
+  if constexpr (Small::EPB < Tile<SHAPE, RULE, FORM, KT, 0>::EPB) {
+    int dev = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess) return err;
+    if (g.nElements <= (int64_t)2 * sms * Small::EPB)
+      return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, SMALL_TILE>(g, st);
   }
   if (g.tileVariant == 1) return launch_assemble_variant<SHAPE, RULE, FORM, KT, ffTile, 1>(g, st);
   if constexpr (Tile<SHAPE, RULE, FORM, KT, 2>::MINB != Tile<SHAPE, RULE, FORM, KT, 0>::MINB) {
