@@ -103,8 +103,7 @@ class GPUAssembler:
             offset += len(g.conn)
         self.nElements = offset
         self._groups_c = (L.EfeGroup * len(structs))(*structs)
-        # default tile (autotune.default_variant): the tensor-core tangent where it measured faster;
-        # the autotuner may choose otherwise
+        # default tile (autotune.default_variant); the autotuner may choose otherwise
         from .autotune import default_variant
 
         for i in range(len(self.groups)):
@@ -256,7 +255,7 @@ class GPUAssembler:
         """Raise CutbackRequest if a material point failed in the last pass (synchronises)."""
         st = self.status.cpu().numpy()
         if st[0] & L.EFE_STATUS_TC_TIMEOUT:
-            raise RuntimeError("the tensor-core tangent gave up waiting for its MMAs (tile variant 3): K is incomplete")
+            raise RuntimeError("the element pass gave up waiting inside a kernel: K is incomplete")
         if st[0] & L.EFE_STATUS_BOUNDS:
             raise IndexError(f"device bounds check: element {0x7FFFFFFF - int(st[1])} indexes outside a node, DOF "
                              "or CSR array (the access was skipped; P, F and K of this pass are invalid)")

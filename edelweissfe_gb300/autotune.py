@@ -9,13 +9,13 @@ import os
 import torch
 
 VARIANTS = (0, 1, 2)
-TENSOR_VARIANT = 3  # the element tangent on the tensor cores (Hexa20 3x3x3 TL Neo-Hooke, FP32 tangent)
+TENSOR_VARIANT = 3  # Hexa20 3x3x3 with an FP32 tangent (once a tensor-core tile; now the two-element tile, as 0-2)
 
 
 def variants_for(asm, gi):
-    """Tile variants to time for group gi: the CTA shapes 0-2, and the tensor-core tangent where the
-    library has it (Hexa20 3x3x3, total-Lagrangian with a hyperelastic material, with an FP32
-    tangent; small-strain Hexa20 takes the number too and runs its one SIMT tile under each)."""
+    """Tile variants to time for group gi: the CTA shapes 0-2, and 3 for Hexa20 3x3x3 with an FP32 tangent
+    (total-Lagrangian with a hyperelastic material, or small strain), which runs its one tile under
+    each number."""
     from . import _lib as L
     from .library import element_type
 
@@ -29,9 +29,8 @@ def variants_for(asm, gi):
 
 
 def default_variant(asm, gi):
-    """Tile variant of group gi before (or without) autotuning: the tensor-core tangent for total-
-    Lagrangian Hexa20 groups (faster than the SIMT tiles in both FP32-tangent modes), else 0.  Small-
-    strain Hexa20 groups run the same tile under every number."""
+    """Tile variant of group gi before (or without) autotuning: 0, or 3 for Hexa20 3x3x3 groups with an
+    FP32 tangent, where the number makes no difference to the tile that runs."""
     from . import _lib as L
     from .library import element_type
 

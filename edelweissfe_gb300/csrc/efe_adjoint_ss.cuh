@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
   if (live) {
     const double* gp = a.geomG + e0 * NQ + pl;
 #pragma unroll 10
-    for (int r = 0; r < NDOF; ++r) tc::cp_async8(sGd + r * NPS + pl, gp + (int64_t)r * stride);
+    for (int r = 0; r < NDOF; ++r) cp_async8(sGd + r * NPS + pl, gp + (int64_t)r * stride);
   }
   for (int t = threadIdx.x; t < 4 * EPB; t += NT) sem[t] = 0;
   __syncthreads();
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
     atomicMax(sem + le * 4, eu);
     atomicMax(sem + le * 4 + 1, ep);
   }
-  tc::cp_async_wait_all();
+  cp_async_wait_all();
   __syncthreads();
   for (int t = threadIdx.x; t < 2 * nLoc * NDOF; t += NT) {
     const int w = t >= nLoc * NDOF, k = t - w * nLoc * NDOF;

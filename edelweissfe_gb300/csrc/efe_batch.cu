@@ -36,14 +36,6 @@ template <typename KT> struct TypeOf<1, KT> : TypeOfBase<EFE_HEXA20, EFE_RULE_3D
 template <typename KT> struct TypeOf<2, KT> : TypeOfBase<EFE_HEXA8, EFE_RULE_3D_2X2X2, TLH, KT, 2> {};
 template <typename KT> struct TypeOf<3, KT> : TypeOfBase<EFE_HEXA8, EFE_RULE_3D_2X2X2, SS3, KT, 3> {};
 template <typename KT> struct TypeOf<4, KT> : TypeOfBase<EFE_QUAD8, EFE_RULE_2D_2X2, TLH, KT, 4> {};
-// type 0 with its tangent on the tensor cores (tile variant 3, efe_hexa20_tc.cuh; FP32 tangent only)
-template <> struct TypeOf<5, float> {
-  using T = PersistentType<EFE_HEXA20, EFE_RULE_3D_3X3X3, TLH, 1, true>;
-  static constexpr size_t bytes = H20TCLayout<false>::bytes;
-  static_assert(H20TCLayout<false>::bytes == H20TCLayout<true>::bytes, "one tile size for both forms");
-  static constexpr int NT = 128, SRC = 0;
-};
-
 constexpr size_t max_of(std::initializer_list<size_t> v) {
   size_t m = 0;
   for (size_t x : v) m = x > m ? x : m;
@@ -71,12 +63,7 @@ cudaError_t run_list(const GroupArgs (*groups)[MAX_PERSISTENT_GROUPS], const int
   int dev = 0, sms = 0, perSM = 0;
   if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
   if ((err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
-  // a list with a tensor-core type allocates TMEM (the runtime's occupancy query then answers 1)
-  if constexpr ((TypeOf<IDX, KT>::T::TC || ...)) {
-    if ((err = resident_ctas_tmem(kern, NT, bytes, (int)H20TC::TMEM_COLS, &perSM)) != cudaSuccess) return err;
-  } else {
-    if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, NT, bytes)) != cudaSuccess) return err;
-  }
+  if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, NT, bytes)) != cudaSuccess) return err;
   if (perSM < 1) return cudaErrorInvalidConfiguration;
   GroupTables<N> tabs;
   int64_t tiles = 0;
@@ -91,14 +78,13 @@ cudaError_t run_list(const GroupArgs (*groups)[MAX_PERSISTENT_GROUPS], const int
   if (tiles + grid > maxTiles) return cudaErrorInvalidValue;
   if ((err = cudaMemsetAsync(counter, 0, sizeof(CT), st)) != cudaSuccess) return err;
   if (grid == 0) return cudaSuccess;
-  kern<<<(unsigned)grid, NT, bytes, st>>>(tabs, counter, sms);
+  kern<<<(unsigned)grid, NT, bytes, st>>>(tabs, counter);
   return cudaGetLastError();
 }
 
 // The smallest instantiated type list covering the types present: total-Lagrangian Neo-Hooke Hexa20
-// + Quad8 (batches of uneven 2D/3D meshes; with the FP32 tangent and every Hexa20 group on tile
-// variant 3, the Hexa20 tangent on the tensor cores), Hexa8 small strain alone (load cases of one
-// material, four CTAs per SM as tile variant 2), or all five types.
+// + Quad8 (batches of uneven 2D/3D meshes; four CTAs per SM with an FP32 tangent), Hexa8 small strain alone (load
+// cases of one material, four CTAs per SM as tile variant 2), or all five types.
 template <typename KT, bool FF, typename CT>
 cudaError_t run_groups(const GroupArgs (*groups)[MAX_PERSISTENT_GROUPS], const int* nGroups, CT* counter,
                        int64_t maxTiles, int64_t* needed, cudaStream_t st) {
@@ -108,13 +94,7 @@ cudaError_t run_groups(const GroupArgs (*groups)[MAX_PERSISTENT_GROUPS], const i
     if (nGroups[k] > 0) present |= 1u << k;
   }
   if ((present & ~((1u << 0) | (1u << 4))) == 0) {
-    if constexpr (std::is_same<KT, float>::value) {
-      // the Hexa20 groups' tangent on the tensor cores when the tile choice says so for all of them
-      bool tc = nGroups[0] > 0;
-      for (int k = 0; k < nGroups[0]; ++k) tc = tc && groups[0][k].tileVariant == 3;
-      if (tc) return run_list<KT, FF, CT, 3, 5, 4>(groups, nGroups, counter, maxTiles, needed, st);
-    }
-    return run_list<KT, FF, CT, 1, 0, 4>(groups, nGroups, counter, maxTiles, needed, st);
+    return run_list<KT, FF, CT, std::is_same<KT, float>::value ? 4 : 1, 0, 4>(groups, nGroups, counter, maxTiles, needed, st);
   }
   if ((present & ~(1u << 3)) == 0) return run_list<KT, FF, CT, 4, 3>(groups, nGroups, counter, maxTiles, needed, st);
   return run_list<KT, FF, CT, 2, 0, 1, 2, 3, 4>(groups, nGroups, counter, maxTiles, needed, st);

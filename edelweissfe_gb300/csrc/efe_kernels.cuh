@@ -17,7 +17,7 @@
 
 #include "efe_device.cuh"
 #include "efe_fixed.cuh"
-#include "efe_tc.cuh"
+#include "efe_async.cuh"
 
 namespace efe {
 
@@ -197,19 +197,6 @@ __device__ __forceinline__ void kadd(KT* p, KT v) {
   atomicAdd(p, v);
 }
 
-// State of the tensor-core tangent across the tiles of one CTA: the base of its TMEM columns and
-// the parity of the MMA-completion mbarrier's next phase.
-struct TCState {
-  uint32_t tmem;
-  uint32_t phase;
-  bool failed;
-  uint64_t* mbar;  // static shared memory of the kernel (never inside a tile's dynamic layout)
-};
-
-// Wait limit of the tensor-core completion (polls of mbarrier.try_wait); far beyond the ~1 us an
-// MMA chunk takes.  On expiry the CTA records EFE_STATUS_TC_TIMEOUT and stops issuing MMAs.
-constexpr int TC_WAIT_LIMIT = 1 << 22;
-
 }  // namespace efe
 
 #include "efe_ss3.cuh"
@@ -222,7 +209,7 @@ __host__ __device__ constexpr bool ss3_warp_tile() {
   return SHAPE == EFE_HEXA8 && RULE == EFE_RULE_3D_2X2X2 && std::is_same<KT, float>::value;
 }
 
-// Hexa20 3x3x3 with an FP32 tangent: two elements on four warps
+// Hexa20 3x3x3 with an FP32 tangent: two elements on four warps (small strain and total-Lagrangian Neo-Hooke)
 template <int SHAPE, int RULE, typename KT>
 __host__ __device__ constexpr bool ss3_hexa20_tile() {
   return SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && std::is_same<KT, float>::value;
@@ -243,9 +230,11 @@ __device__ __forceinline__ void assemble_tile(const GroupArgs& g, const int64_t 
     if constexpr (ss3_warp_tile<SHAPE, RULE, KT>())
       assemble_tile_ss3_hexa8<NT>(g, e0, smem);
     else if constexpr (ss3_hexa20_tile<SHAPE, RULE, KT>())
-      assemble_tile_ss3_hexa20(g, e0, smem);
+      assemble_tile_hexa20<false>(g, e0, smem);
     else
       assemble_tile_ss3<SHAPE, RULE, KT, EPB, NT>(g, e0, smem);
+  } else if constexpr (FORM == TLH && ss3_hexa20_tile<SHAPE, RULE, KT>()) {
+    assemble_tile_hexa20<true>(g, e0, smem);
   } else {
   using L = Layout<SHAPE, RULE, FORM, KT, EPB>;
   constexpr int DIM = L::DIM, NN = L::NN, NQ = L::NQ, NVEC = L::NVEC, NDOF = L::NDOF;
@@ -832,59 +821,6 @@ __global__ void __launch_bounds__(NT, MINB) assemble_kernel(GroupArgs g) {
   assemble_tile<SHAPE, RULE, FORM, KT, EPB, NT, FF>(g, (int64_t)blockIdx.x * EPB, smem);
 }
 
-// Set-up and tear-down of the tensor-core state of a CTA (every thread calls both): the mbarrier
-// of MMA completion, 64 TMEM columns (two 128 x 32 FP32 accumulators) allocated by warp 0; at the
-// end, after a bounded wait for MMAs still in flight if a wait expired, warp 0 frees the columns.
-}  // namespace efe
-
-#include "efe_hexa20_tc.cuh"
-
-namespace efe {
-
-// Set-up and tear-down of the tensor-core state of a CTA (every thread calls both): the mbarrier
-// of MMA completion and H20TC::TMEM_COLS TMEM columns allocated by warp 0; at the end, after a
-// bounded wait for MMAs still in flight if a wait expired, warp 0 frees the columns.
-__device__ __forceinline__ TCState tc_begin(uint64_t* mbar, uint32_t* slot) {
-  if (threadIdx.x == 0) tc::mbar_init(mbar, 1);
-  if (threadIdx.x < 32) tc::tmem_alloc(slot, H20TC::TMEM_COLS);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  return TCState{*slot, 0u, false, mbar};
-}
-__device__ __forceinline__ void tc_end(TCState& tcs) {
-  if (tcs.failed) tc::mbar_wait(tcs.mbar, tcs.phase, TC_WAIT_LIMIT);
-  tc::fence_before_sync();
-  __syncthreads();
-  if (threadIdx.x < 32) tc::tmem_dealloc(tcs.tmem, H20TC::TMEM_COLS);
-}
-
-// Tile variant 3, the Hexa20 3x3x3 total-Lagrangian Neo-Hooke pass with the tensor-core tangent (efe_hexa20_tc.cuh): a grid of resident CTAs (sms per wave), one element per tile, tiles strided by
-// the grid; each CTA allocates its TMEM columns once and frees them at the end.  The CTAs of one
-// wave share no SM, so the wave index picks the warp of the per-point update.  Each element's
-// K_e scatter runs during the next element's material update (the last one after the loop).
-template <bool FF>
-__global__ void __launch_bounds__(128, 3) assemble_kernel_tc(GroupArgs g, int sms) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint64_t mbar;
-  __shared__ uint32_t slot;
-  TCState tcs = tc_begin(&mbar, &slot);
-  int rot = (int)(blockIdx.x / (unsigned)sms), par = 0;
-  int64_t prev = H20TC_DEFER_NONE;  // the element whose K_e is pending in shared memory
-  for (int64_t e = blockIdx.x; e < g.nElements; e += gridDim.x, ++rot, par ^= 1) {
-    const int64_t next = e + gridDim.x < g.nElements ? e + gridDim.x : -1;
-    assemble_tile_h20tc<FF>(g, e, smem, tcs, rot, prev, next, prev >= 0, par);
-    prev = e;
-    __syncthreads();
-  }
-  if (prev >= 0 && !tcs.failed) {
-    using L = H20TCLayout<FF>;
-    h20tc_scatter(g, prev, smem + L::tc_off, reinterpret_cast<const int*>(smem + L::ps_off) + (par ^ 1) * H20TC::NN * H20TC::NN,
-                 reinterpret_cast<const int*>(smem + L::rl_off) + (par ^ 1) * H20TC::NN, threadIdx.x, 128);
-  }
-  tc_end(tcs);
-}
-
 // Groups of one element type for the persistent pass: group k owns the tiles
 // [tileStart[k], tileStart[k+1]) of its type.  Passed by value (kernel parameters).
 constexpr int MAX_PERSISTENT_GROUPS = EFE_PERSISTENT_MAX_GROUPS;
@@ -904,12 +840,10 @@ struct GroupTable {
   int n;
 };
 
-// One element type of the persistent pass: shape, quadrature rule, form, elements per tile and
-// whether its tangent runs on the tensor cores.
-template <int SHAPE_, int RULE_, int FORM_, int EPB_, bool TC_ = false>
+// One element type of the persistent pass: shape, quadrature rule, form and elements per tile.
+template <int SHAPE_, int RULE_, int FORM_, int EPB_>
 struct PersistentType {
   static constexpr int SHAPE = SHAPE_, RULE = RULE_, FORM = FORM_, EPB = EPB_;
-  static constexpr bool TC = TC_;
 };
 
 // The group tables of every type of one persistent launch (kernel parameters).
@@ -921,23 +855,18 @@ struct GroupTables {
 // Run tile t of the concatenated tile ranges of types I, I+1, ... (in the order of the type list) and
 // return true, or return false when t lies past the last type's tiles.
 template <typename KT, int NT, bool FF, int N, int I, typename T0, typename... Rest>
-__device__ __forceinline__ bool persistent_tile(const GroupTables<N>& tabs, long long t, unsigned char* smem,
-                                                TCState* tcs, int rot) {
+__device__ __forceinline__ bool persistent_tile(const GroupTables<N>& tabs, long long t, unsigned char* smem) {
   const GroupTable& tb = tabs.t[I];
   const long long tiles = tb.tileStart[tb.n];
   if (t < tiles) {
     int k = 0;
     while (t >= tb.tileStart[k + 1]) ++k;
-    if constexpr (T0::TC)
-      assemble_tile_h20tc<FF>(tb.g[k], (int64_t)(t - tb.tileStart[k]), smem, *tcs, rot, H20TC_NOW, -1, false,
-                                          0);
-    else
-      assemble_tile<T0::SHAPE, T0::RULE, T0::FORM, KT, T0::EPB, NT, FF>(tb.g[k], (int64_t)(t - tb.tileStart[k]) * T0::EPB,
-                                                                        smem);
+    assemble_tile<T0::SHAPE, T0::RULE, T0::FORM, KT, T0::EPB, NT, FF>(tb.g[k], (int64_t)(t - tb.tileStart[k]) * T0::EPB,
+                                                                      smem);
     return true;
   }
   if constexpr (sizeof...(Rest) > 0)
-    return persistent_tile<KT, NT, FF, N, I + 1, Rest...>(tabs, t - tiles, smem, tcs, rot);
+    return persistent_tile<KT, NT, FF, N, I + 1, Rest...>(tabs, t - tiles, smem);
   else
     return false;
 }
@@ -948,25 +877,18 @@ __device__ __forceinline__ bool persistent_tile(const GroupTables<N>& tabs, long
 // the register budget is held to.  FF: the float-float forms (mixed-ff) of the types that have one.
 template <typename KT, int NT, int MINB, bool FF, typename CT, typename... Types>
 __global__ void __launch_bounds__(NT, MINB)
-    assemble_persistent_kernel(GroupTables<sizeof...(Types)> tabs, CT* counter, int sms) {
+    assemble_persistent_kernel(GroupTables<sizeof...(Types)> tabs, CT* counter) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ long long tile;
-  constexpr bool anyTC = (Types::TC || ...);
-  __shared__ uint64_t mbar;
-  __shared__ uint32_t slot;
-  TCState tcs{};
-  if constexpr (anyTC) tcs = tc_begin(&mbar, &slot);
   while (true) {
     if (threadIdx.x == 0) tile = (long long)atomicAdd(counter, (CT)1);
     __syncthreads();
     const long long t = tile;
     __syncthreads();
-    if (!persistent_tile<KT, NT, FF, (int)sizeof...(Types), 0, Types...>(tabs, t, smem, &tcs,
-                                                                         (int)(blockIdx.x / (unsigned)sms + t)))
+    if (!persistent_tile<KT, NT, FF, (int)sizeof...(Types), 0, Types...>(tabs, t, smem))
       break;
     __syncthreads();
   }
-  if constexpr (anyTC) tc_end(tcs);
 }
 
 }  // namespace efe

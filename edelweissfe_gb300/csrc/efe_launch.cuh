@@ -38,16 +38,20 @@ struct WarpTile {
   static constexpr int NT = VARIANT == SMALL_TILE ? 32 : 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = VARIANT == SMALL_TILE ? 1 : 6;
   static constexpr size_t bytes = SS3Hexa8Layout<NT>::bytes;
 };
-// The two-element tile of small-strain Hexa20 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: five CTAs per
-// SM (96 registers); four (128) or six (80, 116 B of spills) run in 1.06 and 1.07 times its time.
+// The two-element tile of Hexa20 3x3x3 with an FP32 tangent (efe_ss3.cuh), one shape for all variants, the number 3 of the
+// former tensor-core tile among them: five CTAs per SM (96 registers).  Small strain, 13824 elements: four (128 registers)
+// or six (80, 116 B of spills) run in 1.06 and 1.07 times its time; total Lagrangian, 2730 elements: four in 1.14.
+template <bool TL>
 struct Hexa20Tile {
-  static constexpr int NT = SS3Hexa20Layout::NT, EPB = SS3Hexa20Layout::EPB, MINB = 5;
-  static constexpr size_t bytes = SS3Hexa20Layout::bytes;
+  static constexpr int NT = Hexa20Layout<TL>::NT, EPB = Hexa20Layout<TL>::EPB, MINB = 5;
+  static constexpr size_t bytes = Hexa20Layout<TL>::bytes;
 };
 template <int SHAPE, int RULE, int FORM, typename KT, int VARIANT = 0>
-struct Tile : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile<VARIANT>,
-                               typename std::conditional<FORM == SS3 && ss3_hexa20_tile<SHAPE, RULE, KT>(), Hexa20Tile,
-                                                         TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type>::type {};
+struct Tile
+    : std::conditional<FORM == SS3 && ss3_warp_tile<SHAPE, RULE, KT>(), WarpTile<VARIANT>,
+                       typename std::conditional<(FORM == SS3 || FORM == TLH) && ss3_hexa20_tile<SHAPE, RULE, KT>(),
+                                                 Hexa20Tile<FORM == TLH>,
+                                                 TileOf<SHAPE, RULE, FORM, KT, VARIANT>>::type>::type {};
 
 template <int SHAPE, int RULE, int FORM, typename KT, bool FF, int VARIANT>
 cudaError_t launch_assemble_variant(const GroupArgs& g, cudaStream_t st) {
@@ -62,70 +66,10 @@ cudaError_t launch_assemble_variant(const GroupArgs& g, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// the tensor-core tangent (tile variant 3) exists for the Hexa20 3x3x3 total-Lagrangian Neo-Hooke form with an FP32
-// tangent; on small-strain Hexa20 variant 3 names the two-element tile too, which runs in 372 us where a tensor-core tile
-// took 678 (13824 elements, von Mises): its FP64 return map on one warp at a time and its twelve warps per SM
-// bound that one
-template <int SHAPE, int RULE, int FORM, typename KT>
-constexpr bool has_tc_variant() {
-  return SHAPE == EFE_HEXA20 && RULE == EFE_RULE_3D_3X3X3 && FORM == TLH && std::is_same<KT, float>::value;
-}
-
-// Resident CTAs per SM of a kernel that allocates tmemCols TMEM columns per CTA, from its registers
-// (allocated per thread in units of 8), its shared memory (plus the per-CTA reservation), its threads
-// and the SM's 512 TMEM columns.  The runtime's occupancy query answers 1 for kernels that allocate
-// TMEM whatever their size; the CTAs beyond what actually fits only wait for an SM (none waits on
-// another, and tcgen05.alloc waits for free columns), so an estimate that is too high costs nothing.
-template <typename K>
-cudaError_t resident_ctas_tmem(K kern, int nt, size_t dynBytes, int tmemCols, int* perSM) {
-  cudaFuncAttributes fa;
-  cudaError_t err = cudaFuncGetAttributes(&fa, kern);
-  if (err != cudaSuccess) return err;
-  int dev = 0, regsSM = 0, smemSM = 0, reserved = 0, threadsSM = 0;
-  if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
-  if ((err = cudaDeviceGetAttribute(&regsSM, cudaDevAttrMaxRegistersPerMultiprocessor, dev)) != cudaSuccess) return err;
-  if ((err = cudaDeviceGetAttribute(&smemSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return err;
-  if ((err = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess) return err;
-  if ((err = cudaDeviceGetAttribute(&threadsSM, cudaDevAttrMaxThreadsPerMultiProcessor, dev)) != cudaSuccess) return err;
-  const int regs = (fa.numRegs + 7) / 8 * 8;
-  int n = regsSM / (regs * nt);
-  const long long perCta = (long long)dynBytes + (long long)fa.sharedSizeBytes + reserved;
-  n = std::min<long long>(n, smemSM / perCta);
-  n = std::min(n, threadsSM / nt);
-  n = std::min(n, 512 / tmemCols);
-  *perSM = n;
-  return n >= 1 ? cudaSuccess : cudaErrorInvalidConfiguration;
-}
-
-template <bool FF>
-cudaError_t launch_assemble_tc(const GroupArgs& g, cudaStream_t st) {
-  constexpr int NT = 128;
-  constexpr size_t bytes = H20TCLayout<FF>::bytes;
-  static_assert(bytes <= 74 * 1024, "three tensor-core tiles must fit in one SM");
-  auto kern = assemble_kernel_tc<FF>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess) return err;
-  // the largest shared-memory partition: without it the occupancy query (and the launch) assume the
-  // default split and fit one CTA per SM
-  err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-  if (err != cudaSuccess) return err;
-  int dev = 0, sms = 0, perSM = 0;
-  if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
-  if ((err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
-  if ((err = resident_ctas_tmem(kern, NT, bytes, (int)H20TC::TMEM_COLS, &perSM)) != cudaSuccess) return err;
-  int64_t grid = (int64_t)sms * perSM;
-  if (grid > g.nElements) grid = g.nElements;
-  if (grid == 0) return cudaSuccess;
-  kern<<<(unsigned)grid, NT, bytes, st>>>(g, sms);
-  return cudaGetLastError();
-}
-
 template <int SHAPE, int RULE, int FORM, typename KT, bool FF = false>
 cudaError_t launch_assemble(const GroupArgs& g, cudaStream_t st) {
-  constexpr bool ffTile = FF && FORM != SS3;  // the small-strain solids form their B-products in integers in either mode
-  if constexpr (has_tc_variant<SHAPE, RULE, FORM, KT>()) {
-    if (g.tileVariant == 3) return launch_assemble_tc<FF>(g, st);
-  }
+  // the small-strain solids and the Hexa20 tile form their B-products in integers in either mode
+  constexpr bool ffTile = FF && FORM != SS3 && !(FORM == TLH && ss3_hexa20_tile<SHAPE, RULE, KT>());
   // A small group's ordinary tiles leave most SMs without one, and a tile's phases one after the other are then the
   // whole time: small tiles up to two per SM.  320 CPE4 elements (fp64) 11 us against 19, 1200 CPE8R 20 against 45, 512
   // C3D8TL (mixed) 15 against 19, 1000 C3D8 (mixed) 18.4 against 19.5; beyond, 1000 C3D8 (fp64) 32 against 28 and 4000 CPE4

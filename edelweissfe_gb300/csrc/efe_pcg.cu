@@ -78,14 +78,14 @@ __device__ __forceinline__ void ff_madd(float& h, float& l, float k, float xh, f
 
 // ---------------------------------------------------------------- copies
 __device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_addr(bar)), "r"(bytes) : "memory");
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
 // global -> shared, both 16-byte aligned, bytes a multiple of 16; policy: the L2 eviction priority
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
-          tc::smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(tc::smem_addr(bar)), "l"(policy)
+          smem_addr(dst)),
+      "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(policy)
       : "memory");
 }
 
@@ -125,7 +125,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __device__ __forceinline__ void store_remote(double* p, int cta, double v) {
   uint32_t addr;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(tc::smem_addr(p)), "r"(cta));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_addr(p)), "r"(cta));
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 // Sum over the slots of all CTAs in slot order by a warp (every lane gets it); false: gave up.  The caller has
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) pcg_kernel(CgArgs a) {
   const int stageBytes = a.capK + a.capC;
   const int stage0 = wid * stageBytes;
   uint64_t* bar = bars + wid;
-  if (lane == 0) tc::mbar_init(bar, 1);
+  if (lane == 0) mbar_init(bar, 1);
   if (tid == 0) shDead = 0;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) pcg_kernel(CgArgs a) {
       sum.zero();
       if (d.staged) {
         if (!landed) {
-          if (!dead && !tc::mbar_wait(bar, phase, COPY_LIMIT)) dead = true;
+          if (!dead && !mbar_wait(bar, phase, COPY_LIMIT)) dead = true;
           phase ^= 1u;
           landed = resident;
         }
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) pcg_kernel(CgArgs a) {
     }
     __syncthreads();
     if (shDead) {  // gave up: let the copy land before the CTA ends
-      if (!resident && w0 < nChunks && d.staged) tc::mbar_wait(bar, phase, COPY_LIMIT);
+      if (!resident && w0 < nChunks && d.staged) mbar_wait(bar, phase, COPY_LIMIT);
       break;
     }
   }

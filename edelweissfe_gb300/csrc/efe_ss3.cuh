@@ -1,5 +1,6 @@
-// efe_ss3.cuh -- the small-strain solid element pass (von Mises, linear elastic; Hexa8, Hexa20) with its
-// B-products in fixed-point integers (efe_fixed.cuh); included by efe_kernels.cuh.
+// efe_ss3.cuh -- the small-strain solid element pass (von Mises, linear elastic; Hexa8, Hexa20), and the total-Lagrangian
+// Neo-Hooke one of Hexa20 3x3x3 with an FP32 tangent, with their B-products in fixed-point integers (efe_fixed.cuh);
+// included by efe_kernels.cuh.
 //
 // What is left to the FP64 pipe, which bound this pass in every mode, is the material update (92 instructions per point,
 // 53 with an FP32 tangent).  The strain increment de = B dU (9 products per node and point), the residual
@@ -14,7 +15,7 @@
 //
 // Measured, von Mises plastic increment, kernel time before (FP64 sums) and with integers: C3D8, FP64 tangent, 31713
 // elements 1027 -> 362 us; FP32 tangent, 262144 elements 1318 -> 995 us; C3D20, FP64 tangent, 2448 elements 1638 -> 325
-// us; FP32 tangent, 13824 elements 678 -> 372 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
+// us; FP32 tangent, 13824 elements 678 -> 380 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
 // -> 2.2e-15, K 7.2e-16 -> 7.1e-16; C3D20 P 5.4e-15 -> 5.3e-15, K 1.89e-15 -> 1.88e-15; FP32 K 6.1e-8 in both.
 //
 // FP64 tangent: K_ab = sum_q  c12 s G_a (x) G_b + c44 s (G_b (x) G_a + G_a . G_b I) - a s nG_a (x) nG_b.  The
@@ -654,32 +655,105 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Hexa20 with 3x3x3 points and an FP32 tangent: two elements on four warps.  A point's row of shared memory holds the
-// digits of dN/dX and then, in their place, the tangent's vectors; a thread forms the blocks of 2 x 2 nodes (14 loads of
-// shared memory for 138 arithmetic instructions per point), and K_e goes to the CSR rows through shared memory, so that
-// the lanes of a warp share the sectors that L2 adds to (the adds alone: 110 us on 13824 elements, 264 us by node pairs).
-// 372 us; the issue slots (63 % used) and the waits of the phases with a thread per point bind it.
-struct SS3Hexa20Layout {
+// Hexa20 with 3x3x3 points and an FP32 tangent, small strain or (TL) total-Lagrangian Neo-Hooke: two elements on four
+// warps.  A point's row of shared memory holds the digits of dN/dX and then, in their place, the tangent's vectors; a
+// thread forms the blocks of 2 x 2 nodes (14 loads of shared memory for 174 arithmetic instructions per point), and K_e goes
+// to the CSR rows through shared memory, so that the lanes of a warp share the sectors that L2 adds to (the adds alone: 110
+// us on 13824 elements, 264 us by node pairs).
+//
+// The Neo-Hooke tangent (displacementtlelement/element.py:408-412) takes two vectors per node too, h = F^-T dN/dX and
+// g = F dN/dX: with c1 = sB and c3 = c4 in every variant, B h = g and dN_a/dX . dN_b/dX = h_a . g_b,
+//   K_ab[j][k] = sum_q s (c2 h_a[j] h_b[k] + c3 (g_a[j] h_b[k] + h_a[j] g_b[k]) - sI h_a[k] h_b[j] + c1 delta_jk h_a . g_b).
+//
+// 13824 elements: small strain (von Mises) 678 -> 380 us, where a tensor-core tile (tcgen05, TF32 hi/lo) ran; TL 704 ->
+// 467 us, mixed-ff 665 -> 468 us, against the same.  That tile's serial phases (operand conversion, FP64 update on one
+// warp, MMA waits) with twelve warps per SM bound it, not the products; its tangent was 8e-7 off, this one 7e-8.  Here
+// the issue slots (63 % used, small strain) and the waits of the phases with a thread per point bind.
+template <bool TL>
+struct Hexa20Layout {
   static constexpr int EPB = 2, NT = 128, NN = 20, NQ = 27, NDOF = 60, NP = EPB * NQ, NB = 55;  // NB: node blocks A <= B
   // a point's row in doublewords: 60 digits, then the floats (dN/dX, n dN/dX) of 20 nodes; odd
-  static constexpr int SV = 61, DS = 7, SK = 61;
+  static constexpr int SV = 61, DS = TL ? 9 : 7, SN = TL ? 19 : 7, SK = 61;
   static constexpr size_t v_off = 0;                            // fx [NP][SV]
   static constexpr size_t u_off = v_off + 8 * NP * SV;          // fx [EPB][NDOF]
-  static constexpr size_t d_off = u_off + 8 * EPB * NDOF;       // int64 [NP][DS]: half of the strain; fx: s sigma
+  static constexpr size_t d_off = u_off + 8 * EPB * NDOF;       // int64 [NP][DS]: half of the strain (H); fx: s sigma (s P)
   static constexpr size_t k_bytes = 4 * EPB * NDOF * SK;        // K_e, in their place: float [EPB][NDOF][SK]
   static_assert(k_bytes <= d_off + 8 * NP * DS, "K_e fits the area of the operands");
-  static constexpr size_t c_off = (d_off + 8 * NP * DS + 15) / 16 * 16;  // float4 [NP]: coefficients, unit of the upper digits
-  static constexpr size_t n_off = c_off + 16 * NP;              // float [NP][DS]: flow direction
-  static constexpr size_t mc_off = (n_off + 4 * NP * DS + 15) / 16 * 16;  // VMConst [EPB]
+  static constexpr size_t c_off = (d_off + 8 * NP * DS + 15) / 16 * 16;  // float4 [NP]: coefficients (small strain: and the unit)
+  // float [NP][SN]: flow direction, or F^-1, F and the unit of the upper digits
+  static constexpr size_t n_off = c_off + 16 * NP;
+  static constexpr size_t mc_off = (n_off + 4 * NP * SN + 15) / 16 * 16;  // VMConst [EPB]
   static constexpr size_t sl_off = mc_off + sizeof(VMConst) * EPB;        // int [EPB][NN][NN]: pair slots
   static constexpr size_t rl_off = sl_off + 4 * EPB * NN * NN;            // int [EPB][NN]: row lengths
   static constexpr size_t e_off = rl_off + 4 * EPB * NN;                  // int [2][NP]: halves of em_g; [EPB]: em_u, em_s
   static constexpr size_t bytes = e_off + 4 * (2 * NP + 2 * EPB);
 };
 
-__device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
-  using L = SS3Hexa20Layout;
-  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, SV = L::SV, DS = L::DS, EPB = L::EPB, NT = L::NT;
+// Total-Lagrangian Neo-Hooke update of one point from H (displacementtlelement/element.py:386-414): state, strain, s P =
+// s tau F^-T = s sB F + s sI F^-T, and for the tangent c = (c2, c3, -sI, c1) s and n = F^-1, F.
+__device__ __forceinline__ void hexa20_neo_hooke(const GroupArgs& g, int64_t e, int64_t pt, int64_t stride, double s,
+                                                 const double H[9], double sP[9], float4* c, float* n) {
+  const double* props = g.props + e * g.nProps;
+  double F[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) F[i][j] = (i == j ? 1.0 : 0.0) + H[i * 3 + j];
+  // Green-Lagrange E = 1/2 (H + H^T + H^T H) (:386), order 11, 22, 33, 12, 23, 13
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int i = f < 3 ? f : (f == 4 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+    const double E = 0.5 * ((H[i * 3 + j] + H[j * 3 + i]) + (H[i] * H[j] + H[3 + i] * H[3 + j] + H[6 + i] * H[6 + j]));
+    g.auxTemp[(int64_t)f * stride + pt] = E;
+    g.stateTemp[(int64_t)(6 + f) * stride + pt] = f < 3 ? E : 2.0 * E;
+  }
+  double iF[3][3];
+  iF[0][0] = F[1][1] * F[2][2] - F[1][2] * F[2][1];
+  iF[1][0] = F[1][2] * F[2][0] - F[1][0] * F[2][2];
+  iF[2][0] = F[1][0] * F[2][1] - F[1][1] * F[2][0];
+  const double J = F[0][0] * iF[0][0] + F[0][1] * iF[1][0] + F[0][2] * iF[2][0];
+  iF[0][1] = F[0][2] * F[2][1] - F[0][1] * F[2][2];
+  iF[0][2] = F[0][1] * F[1][2] - F[0][2] * F[1][1];
+  iF[1][1] = F[0][0] * F[2][2] - F[0][2] * F[2][0];
+  iF[1][2] = F[0][2] * F[1][0] - F[0][0] * F[1][2];
+  iF[2][1] = F[0][1] * F[2][0] - F[0][0] * F[2][1];
+  iF[2][2] = F[0][0] * F[1][1] - F[0][1] * F[1][0];
+  const double rJ = 1.0 / J;
+  double B[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int i = f < 3 ? f : (f == 4 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+    B[f] = F[i][0] * F[j][0] + F[i][1] * F[j][1] + F[i][2] * F[j][2];
+  }
+  const NeoHookeScalars o =
+      neo_hooke_scalars(g.material, props[0], props[1], J, B[0] + B[1] + B[2], F[0][0] + F[1][1] + F[2][2]);
+  bool finite = true;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const double tau = f < 3 ? o.sB * B[f] + o.sI : o.sB * B[f];
+    g.stateTemp[(int64_t)f * stride + pt] = tau;
+    finite = finite && finite_bits(tau);
+  }
+  g.stateTemp[(int64_t)12 * stride + pt] = o.energy;
+  if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
+  const double aF = s * o.sB, aI = s * o.sI, aIJ = aI * rJ;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      sP[i * 3 + j] = fma(aIJ, iF[j][i], aF * F[i][j]);
+      n[j * 3 + i] = ff_split_rn_bits(iF[j][i] * rJ).h;
+      n[9 + i * 3 + j] = ff_split_rn_bits(F[i][j]).h;
+    }
+  *c = make_float4(ff_split_rn_bits(o.c2 * s).h, ff_split_rn_bits(o.c3 * s).h, ff_split_rn_bits(-aI).h,
+                   ff_split_rn_bits(o.c1 * s).h);
+}
+
+template <bool TL>
+__device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
+  using L = Hexa20Layout<TL>;
+  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, SV = L::SV, DS = L::DS, SN = L::SN, EPB = L::EPB, NT = L::NT;
+  const double* Ux = TL ? g.U : g.dU;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   fx* sv = reinterpret_cast<fx*>(smem + L::v_off);
   fx* su = reinterpret_cast<fx*>(smem + L::u_off);
@@ -696,7 +770,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
   const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB;
   const bool vm = g.material == EFE_MAT_VON_MISES;
 
-  for (int t = tid; t < nLoc * NN * NN; t += NT) tc::cp_async4(sps + t, g.pairSlot + e0 * NN * NN + t);
+  for (int t = tid; t < nLoc * NN * NN; t += NT) cp_async4(sps + t, g.pairSlot + e0 * NN * NN + t);
   // ---- dN/dX: two threads per point, 30 values each; dU relative to the element's first node: warps 0 and 1; the
   // material constants: two lanes of warp 3 that have no points
   {
@@ -724,7 +798,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
           if (in_bounds(g, dof, g.nDof - 2, e) && in_bounds(g, dof0, g.nDof - 2, e)) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-              u[c] = g.dU[dof + c] - g.dU[dof0 + c];
+              u[c] = Ux[dof + c] - Ux[dof0 + c];
               eu = fx_max_exponent(eu, u[c]);
             }
           }
@@ -742,7 +816,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
       for (int i = 0; i < H; ++i) em = fx_max_exponent(em, G[i]);
       sem[part * NP + r] = em;
     }
-    if (wid == 3 && lane >= 32 - nLoc) {
+    if (!TL && wid == 3 && lane >= 32 - nLoc) {
       const int k = 31 - lane;
       smc[k] = vm_const<true>(g.props + (e0 + k) * g.nProps, vm);
     }
@@ -764,33 +838,42 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
   const int eg = live ? max(sem[pr], sem[NP + pr]) : 0;
   const int64_t e = e0 + le, pt = e * NQ + lane;
   const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
-  int64_t st[6];
+  constexpr int NS = TL ? 9 : 6;
+  int64_t st[NS];
   double sig[6], kappa = 0.0, s = 0.0;
   if (live && half == 0) {
+    if constexpr (!TL) {
 #pragma unroll
-    for (int f = 0; f < 6; ++f) sig[f] = g.stateRef[(int64_t)f * stride + pt];
-    if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
+      for (int f = 0; f < 6; ++f) sig[f] = g.stateRef[(int64_t)f * stride + pt];
+      if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
+    }
     s = g.geomS[pt];
   }
   if (live) {
-    FxSum acc[6] = {};
+    FxSum acc[NS] = {};
     const fx *gp = sv + pr * SV + half * 30, *up = su + le * NDOF + half * 30;
 #pragma unroll 5
     for (int a = 0; a < NN / 2; ++a) {
-      const fx ux = up[a * 3], uy = up[a * 3 + 1], uz = up[a * 3 + 2];
-      const fx gx = gp[a * 3], gy = gp[a * 3 + 1], gz = gp[a * 3 + 2];
-      fx_fma(acc[0], gx, ux);
-      fx_fma(acc[1], gy, uy);
-      fx_fma(acc[2], gz, uz);
-      fx_fma(acc[3], gy, ux);
-      fx_fma(acc[3], gx, uy);
-      fx_fma(acc[4], gz, ux);
-      fx_fma(acc[4], gx, uz);
-      fx_fma(acc[5], gz, uy);
-      fx_fma(acc[5], gy, uz);
+      const fx u[3] = {up[a * 3], up[a * 3 + 1], up[a * 3 + 2]}, G[3] = {gp[a * 3], gp[a * 3 + 1], gp[a * 3 + 2]};
+      if constexpr (TL) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) fx_fma(acc[i * 3 + j], u[i], G[j]);
+      } else {
+        fx_fma(acc[0], G[0], u[0]);
+        fx_fma(acc[1], G[1], u[1]);
+        fx_fma(acc[2], G[2], u[2]);
+        fx_fma(acc[3], G[1], u[0]);
+        fx_fma(acc[3], G[0], u[1]);
+        fx_fma(acc[4], G[2], u[0]);
+        fx_fma(acc[4], G[0], u[2]);
+        fx_fma(acc[5], G[2], u[1]);
+        fx_fma(acc[5], G[1], u[2]);
+      }
     }
 #pragma unroll
-    for (int f = 0; f < 6; ++f) {
+    for (int f = 0; f < NS; ++f) {
       st[f] = fx_int(acc[f], -1);
       if (half) sde[pr * DS + f] = st[f];
     }
@@ -800,43 +883,52 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
   // ---- material points: one warp of each element
   if (half == 0) {
     int es = 0;
-    double ss[6] = {0, 0, 0, 0, 0, 0};
+    double ss[NS] = {};  // s sigma, or s P = s tau F^-T
+    // the upper digits of dN/dX have 29 bits, more than a float
+    auto unit = [&] { return eg >= FX_NAN ? __int_as_float(0x7fc00000) : ldexpf(1.0f, max(-300, min(300, eg - 1051))); };
     if (live) {
-      double de[6], eps[6];
+      double de[NS];  // the strain increment, or H
 #pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        de[f] = fx_value(st[f] + sde[pr * DS + f], eg + emu[le] + 1);
-        eps[f] = g.stateRef[(int64_t)(6 + f) * stride + pt];
-      }
-      bool ok = true;
-      TangentF32 T;
-      if (vm)
-        ok = von_mises_3d_f32(smc[le], sig, de, kappa, T);
-      else
-        linear_elastic_3d(smc[le], sig, de, T);
-      bool finite = true;
+      for (int f = 0; f < NS; ++f) de[f] = fx_value(st[f] + sde[pr * DS + f], eg + emu[le] + 1);
+      if constexpr (TL) {
+        sn[pr * SN + 18] = unit();
+        hexa20_neo_hooke(g, e, pt, stride, s, de, ss, sc + pr, sn + pr * SN);
+      } else {
+        double eps[6];
 #pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        g.stateTemp[(int64_t)f * stride + pt] = sig[f];
-        g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
-        finite = finite && finite_bits(sig[f]);
-        ss[f] = s * sig[f];
-        es = fx_max_exponent(es, ss[f]);
-        sn[pr * DS + f] = T.n[f];
+        for (int f = 0; f < 6; ++f) eps[f] = g.stateRef[(int64_t)(6 + f) * stride + pt];
+        bool ok = true;
+        TangentF32 T;
+        if (vm)
+          ok = von_mises_3d_f32(smc[le], sig, de, kappa, T);
+        else
+          linear_elastic_3d(smc[le], sig, de, T);
+        bool finite = true;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+          g.stateTemp[(int64_t)f * stride + pt] = sig[f];
+          g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
+          finite = finite && finite_bits(sig[f]);
+          ss[f] = s * sig[f];
+          es = fx_max_exponent(es, ss[f]);
+          sn[pr * SN + f] = T.n[f];
+        }
+        if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
+        if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
+        if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
+        sc[pr] = make_float4(ff_split_rn_bits(T.c12 * s).h, ff_split_rn_bits(T.c44 * s).h, ff_split_rn_bits(T.a * s).h,
+                             unit());
       }
-      if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
-      if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
-      if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
-      // the upper digits of dN/dX have 29 bits, more than a float
-      const float unit = eg >= FX_NAN ? __int_as_float(0x7fc00000) : ldexpf(1.0f, max(-300, min(300, eg - 1051)));
-      sc[pr] = make_float4(ff_split_rn_bits(T.c12 * s).h, ff_split_rn_bits(T.c44 * s).h, ff_split_rn_bits(T.a * s).h, unit);
+      if constexpr (TL)
+#pragma unroll
+        for (int f = 0; f < NS; ++f) es = fx_max_exponent(es, ss[f]);
       es += eg;
     }
     es = __reduce_max_sync(0xffffffffu, es);
     if (lane == 0) ems[le] = es;
     if (live)
 #pragma unroll
-      for (int f = 0; f < 6; ++f) sd[pr * DS + f] = fx_make(ss[f], es - eg);
+      for (int f = 0; f < NS; ++f) sd[pr * DS + f] = fx_make(ss[f], es - eg);
   }
   __syncthreads();
 
@@ -846,7 +938,8 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
     if (k < NDOF && el < nLoc) {
       const int a = k / 3, c = k - 3 * a;
       const int64_t e = e0 + el;
-      const int v0 = c == 0 ? 0 : c + 2, v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
+      const int v0 = TL ? 3 * c : (c == 0 ? 0 : c + 2), v1 = TL ? 3 * c + 1 : (c == 0 ? 3 : (c == 1 ? 1 : 5)),
+                v2 = TL ? 3 * c + 2 : (c == 0 ? 4 : (c == 1 ? 5 : 2));
       FxSum s[3] = {};  // one for each direction: 27 products
       const fx *gp = sv + el * NQ * SV + a * 3, *dp = sd + el * NQ * DS;
 #pragma unroll 3
@@ -870,18 +963,31 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
 
   // ---- the tangent's vectors in the place of the digits
   if (live) {
-    const float unit = sc[pr].w;
-    float n[6];
+    const float unit = TL ? sn[pr * SN + 18] : sc[pr].w;
+    float n[TL ? 18 : 6];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) n[f] = sn[pr * DS + f];
+    for (int f = 0; f < (TL ? 18 : 6); ++f) n[f] = sn[pr * SN + f];
     fx* row = sv + pr * SV + half * 30;
 #pragma unroll 5
     for (int a = 0; a < NN / 2; ++a) {
       const float gx = (float)row[a * 3].h * unit, gy = (float)row[a * 3 + 1].h * unit, gz = (float)row[a * 3 + 2].h * unit;
+      float x[6];
+      if constexpr (TL) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          x[i] = n[i] * gx + n[3 + i] * gy + n[6 + i] * gz;                    // h = F^-T dN/dX
+          x[3 + i] = n[9 + 3 * i] * gx + n[10 + 3 * i] * gy + n[11 + 3 * i] * gz;  // F dN/dX
+        }
+      } else {
+        x[0] = gx, x[1] = gy, x[2] = gz;
+        x[3] = n[0] * gx + n[3] * gy + n[4] * gz;
+        x[4] = n[3] * gx + n[1] * gy + n[5] * gz;
+        x[5] = n[4] * gx + n[5] * gy + n[2] * gz;
+      }
       float2* v = reinterpret_cast<float2*>(row + a * 3);
-      v[0] = make_float2(gx, gy);
-      v[1] = make_float2(gz, n[0] * gx + n[3] * gy + n[4] * gz);
-      v[2] = make_float2(n[3] * gx + n[1] * gy + n[5] * gz, n[4] * gx + n[5] * gy + n[2] * gz);
+      v[0] = make_float2(x[0], x[1]);
+      v[1] = make_float2(x[2], x[3]);
+      v[2] = make_float2(x[4], x[5]);
     }
   }
   __syncthreads();
@@ -915,15 +1021,15 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
         float lg[3], mg[3], tn[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          lg[j] = c.x * ga[x][j];
-          mg[j] = c.y * ga[x][j];
-          tn[j] = -c.z * na[x][j];
+          lg[j] = TL ? fmaf(c.y, na[x][j], c.x * ga[x][j]) : c.x * ga[x][j];
+          mg[j] = (TL ? c.z : c.y) * ga[x][j];
+          tn[j] = TL ? c.y * ga[x][j] : -c.z * na[x][j];
         }
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
 #pragma unroll
           for (int j = 0; j < 3; ++j) {
-            dot[x][y] = fmaf(mg[j], gb[y][j], dot[x][y]);
+            dot[x][y] = TL ? fmaf(c.w * ga[x][j], nb[y][j], dot[x][y]) : fmaf(mg[j], gb[y][j], dot[x][y]);
 #pragma unroll
             for (int k = 0; k < 3; ++k)
               acc[x][y][j][k] += fmaf(tn[j], nb[y][k], fmaf(mg[k], gb[y][j], lg[j] * gb[y][k]));
@@ -938,7 +1044,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa20(const GroupArgs& g, con
 #pragma unroll
         for (int j = 0; j < 3; ++j) acc[x][y][j][j] += dot[x][y];
   }
-  tc::cp_async_wait_all();
+  cp_async_wait_all();
   __syncthreads();
 
   // ---- K_e[(b, k)][(a, j)] over the operands (the element tangents are symmetric), then a warp per node b: its three

@@ -76,8 +76,8 @@ enum {
   EFE_K_FP32_FF = 2 /* as EFE_K_FP32, and for total-Lagrangian Neo-Hooke F, F^-T dN/dX and the
                      element residual are formed in float-float arithmetic (~48-bit significand,
                      needs geomG32 and geomGlo); the Kirchhoff stress, state and the global
-                     residual accumulation stay FP64 (small-strain solids form their strain and
-                     residual in exact integer sums in every mode)                              */
+                     residual accumulation stay FP64 (small-strain solids and Hexa20 3x3x3 form
+                     their kinematics and residual in exact integer sums in every mode)         */
 };
 /* status words (int32[3], zeroed by the caller): status[0] = OR of EFE_STATUS_* bits,
    status[1] = INT32_MAX - (global index of the first failing element), 0 if none,
@@ -86,8 +86,8 @@ enum {
   EFE_STATUS_CUTBACK = 1,      /* a material point asked for a cutback (CutbackRequest(.., 0.5)) */
   EFE_STATUS_BAD_JACOBIAN = 2, /* det J <= 0 or not finite at set-up                               */
   EFE_STATUS_NONFINITE = 4,    /* a non-finite stress was produced                                 */
-  EFE_STATUS_TC_TIMEOUT = 8,   /* the tensor-core tangent (tile variant 3) gave up waiting for its
-                                  MMAs; K of the pass is incomplete (an internal error)           */
+  EFE_STATUS_TC_TIMEOUT = 8,   /* a pass gave up waiting inside a kernel and its K is incomplete (an
+                                  internal error; no tile of this version waits)                  */
   EFE_STATUS_BOUNDS = 16       /* debug checks (environment EFE_DEVICE_CHECKS=1, read once per
                                   process): a connectivity node outside [0, nNodes), a node DOF
                                   outside the DOF vector, or a pair slot + block offset outside
@@ -137,11 +137,9 @@ typedef struct EfeGroup {
   double* auxTemp;           /* TL only: Green-Lagrange strain of this call                  */
   int32_t tileVariant;       /* CTA shape of the element pass: 0 = 128 threads, 3 CTAs/SM;
                                 1 = 256 threads, larger tiles; 2 = as 0 with 4 CTAs/SM where
-                                shared memory allows; 3 = the element tangent on the tensor
-                                cores (tcgen05, TF32 hi/lo split, FP32 accumulation in TMEM) for
-                                Hexa20 3x3x3 total-Lagrangian Neo-Hooke with an FP32 tangent
-                                (EFE_K_FP32 / EFE_K_FP32_FF), otherwise as 0 (chosen by the
-                                autotuner)                                                     */
+                                shared memory allows; 3 = as 0.  Hexa20 3x3x3 and small-strain
+                                Hexa8 2x2x2 with an FP32 tangent have one tile under every number,
+                                small groups take smaller ones (chosen by the autotuner)       */
 } EfeGroup;
 
 /* One (mesh, group) pair of a persistent launch, with its own DOF vectors and CSR data. */
@@ -226,8 +224,7 @@ int32_t efe_adjoint_small_strain(const EfeMesh* mesh, const EfeGroup* group, con
    EFE_PERSISTENT_MAX_GROUPS groups of each of the types Hexa20 3x3x3 and Hexa8 2x2x2 total-
    Lagrangian Neo-Hooke and small-strain von Mises / linear elastic, and Quad8 2x2 total-Lagrangian
    Neo-Hooke, in any order, precision EFE_K_FP64 / EFE_K_FP32 / EFE_K_FP32_FF (the last needs
-   geomG32 and geomGlo); with an FP32 tangent and tileVariant 3 on every Hexa20 total-Lagrangian
-   group, their tangents run on the tensor cores.  Other types return EFE_ERR_UNSUPPORTED. */
+   geomG32 and geomGlo).  Other types return EFE_ERR_UNSUPPORTED. */
 #define EFE_PERSISTENT_MAX_GROUPS 8
 int32_t efe_compute_elements_persistent(const EfeWorkItem* items, int32_t nItems, int32_t kPrecision,
                                         uint64_t* workCounter, int32_t* status, void* stream);
