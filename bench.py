@@ -151,8 +151,8 @@ def bytes_per_pass(nEl, nQ, nState, nNodes, nDof, nnz, kbytes, nn, dim, state_re
 # (vonmises.py:210-251), residual B^T sigma 72 FMA (element.py:322-344); J, J^-1 and dN/dX are
 # formed once at set-up, as the reference's initializeElement does.  The FP64 mode adds the tangent
 # K_e += B^T C B (C.B 6*3*24 = 432 FMA, B^T (C B) 3*24^2 = 1728 FMA per point, element.py:342); the
-# mixed modes form it in FP32 (not counted here).  In mixed-ff the strain and residual run in
-# float-float on the FP32 pipe, so only the material update stays FP64.
+# mixed modes form it in FP32 (not counted here).  The kernels form all of these sums but the material
+# update in fixed-point integers, so the rate against the FP64 peak can pass 1.
 FP64_FLOP_PER_POINT = {"fp64": 2 * 72 + 150 + 2 * 72 + 2 * (432 + 1728), "mixed": 2 * 72 + 150 + 2 * 72,
                        "mixed-ff": 150}  # fmt: skip
 
@@ -736,7 +736,7 @@ def run_batched(args):
 def run_hexa20tl(args):
     """The C3D20TL Neo-Hooke (a) element pass on an n x n x n/2 box (default n = 32: 16,384 elements)
     under F = I + 0.05 N(0,1): CUDA-event time per pass for each precision with an FP32 tangent and
-    tile variants 0 (SIMT tangent), 2 and 3 (tangent on the tensor cores), and the difference of each
+    tile variants 0, 2 and 3 (one tile under each number), and the difference of each
     variant's K and P from variant 0's."""
     return _run_hexa20(args, "tl")
 
@@ -1184,7 +1184,7 @@ def run_plastic(args):
         "value": 1e3 / timing["kernel_ms"], "unit": "grad/s", "higher_is_better": True,
         "with_adjoint_solves": {"value": 1.0 / bwd_s, "unit": "grad/s", "backward_wall_s": bwd_s},
         "dtype": "f64 residual/state/return map + f32 tangent (mixed); reverse passes: f64 return map, "
-                 "float-float B-products", "data": "synthetic",
+                 "integer B-products", "data": "synthetic",
         "config": {"workload": f"C3D20 von Mises J2 {n}x{n}x{max(1, n // 2)} on [0,2]x[0,2]x[0,1], per-element "
                                "fy0 ~ U[200,300], H ~ U[800,1200], 10 uniaxial increments to 0.5% strain; "
                                "J = total top reaction", "elements": len(conn), "dofs": nDof, "nnz": int(asm.nnz)},
@@ -1331,7 +1331,7 @@ def main():
                                   "hbm": roofline_hbm(abytes, results["mixed-ff"]["kernel_ms"])}},
         "errors": errs,
         "parity": parity,
-        # the roof that binds the pass is the FP64 pipe (ncu: FP64 pipe ~80 % active, DRAM ~13 %);
+        # the FP64 work of the reference's sums against the FP64 peak (the kernel's own FP64: fp64_pipe_active_pct);
         # the HBM fraction of the same launch is kept beside it
         "roofline": {
             "bound": "fp64",
