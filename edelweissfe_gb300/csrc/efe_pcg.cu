@@ -28,6 +28,7 @@
 // 64^3 Hexa8, FP32 values 212 -> 75 us (phase A 55 us for 288 MB, 5.2 TB/s; the two synchronisations 8, B 10),
 // 32^3 Hexa8, FP64 values 56.6 -> 29 us (phase A 16 us, its FP64 work alone 15); 40 x 8 plate 15.4 -> 7.0 us.
 #include "efe_launch.cuh"
+#include "efe_pcg_slots.cuh"
 
 #include <type_traits>
 
@@ -37,9 +38,10 @@ namespace {
 
 // work layout (doubles): [0..1] r.z by iteration parity, [2] r.r, [3] p.Ap, [4] arrival counters,
 // [5] 1 when the solve has ended (-1: a wait gave up), [6] iterations run, [7] 1 when the last test asked to
-// stop, [8 ..) one slot of 16 bytes per CTA and sum
+// stop, [8 ..) the slots (efe_pcg_slots.cuh)
 constexpr int PART0 = 8, MAX_GRID = 512;
-static_assert(PART0 + 4 * 2 * MAX_GRID <= EFE_PCG_WORK_DOUBLES, "work layout");
+static_assert(PART0 + pcg_slots(MAX_GRID) * PCG_SLOT_DOUBLES <= EFE_PCG_WORK_DOUBLES, "work layout");
+static_assert(sizeof(ulonglong2) == PCG_SLOT_DOUBLES * sizeof(double), "a slot");
 constexpr int MAX_WARPS = 16;
 constexpr int MAX_CLUSTER = 8;
 constexpr int BARRIER_LIMIT = 1 << 22;  // polls of another CTA's arrival (about two seconds) before it gives up
@@ -129,7 +131,7 @@ __device__ __forceinline__ void store_remote(double* p, int cta, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 // Sum over the slots of all CTAs in slot order by a warp (every lane gets it); false: gave up.  The caller has
-// seen every CTA arrive, so the values are there or on their way.
+// seen every CTA arrive, so the values are there or on their way, and stay until the caller's own next arrival.
 __device__ __forceinline__ bool gather_sum(const ulonglong2* slots, int nSlots, uint32_t epoch, int lane, double& sum) {
   double v = 0.0;
   bool ok = true;
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) pcg_kernel(CgArgs a) {
   uint32_t phase = 0;  // parity of the copy's next completion
   bool dead = false;   // a wait gave up: no more waits, the kernel runs out
   uint32_t epoch = 0, arrivals = 0, passes = 0;
-  ulonglong2* slots = reinterpret_cast<ulonglong2*>(a.work + PART0);  // three arrays of gridDim slots
+  ulonglong2* slots = reinterpret_cast<ulonglong2*>(a.work + PART0);  // pcg_slots(gridDim) of them
   uint32_t* counters = reinterpret_cast<uint32_t*>(a.work + 4);       // arrivals at the sums, at the barrier
   const int ng = gridDim.x;
   double rz = a.work[a.k0 & 1], rr = 0.0, pAp = 0.0;
@@ -470,14 +472,15 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) pcg_kernel(CgArgs a) {
       if constexpr (CL) {
         if (lane < ng) store_remote(&all[epoch & 1][wid * MAX_CLUSTER + blockIdx.x], lane, s);
       } else {
+        ulonglong2* set = slots + pcg_slot(epoch, wid, ng);
         if (lane == 0) {
-          post(slots + wid * ng + blockIdx.x, s, epoch);
+          post(set + blockIdx.x, s, epoch);
           if (wid == 0) arrive(counters);
           if (!dead && !await(counters, arrivals * ng)) dead = true;
         }
         __syncwarp();
         dead = __shfl_sync(0xffffffffu, (int)dead, 0);
-        if (!dead && !gather_sum(slots + wid * ng, ng, epoch, lane, s)) dead = true;
+        if (!dead && !gather_sum(set, ng, epoch, lane, s)) dead = true;
         if (cross) asm volatile("fence.acq_rel.gpu;" ::: "memory");
         if (lane == 0) {
           sums[wid] = s;
@@ -666,7 +669,7 @@ cudaError_t launch(CgArgs a, int warps, cudaStream_t st) {
   }
   // the counters, and the slots, whose epochs start from 0 in every launch
   if ((e = cudaMemsetAsync(a.work + 4, 0, sizeof(double), st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(a.work + PART0, 0, (size_t)grid * 3 * sizeof(ulonglong2), st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(a.work + PART0, 0, (size_t)pcg_slots((int)grid) * sizeof(ulonglong2), st)) != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kern), dim3((unsigned)grid), dim3(warps * 32), args, bytes, st);
 }
