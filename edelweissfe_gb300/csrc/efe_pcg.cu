@@ -675,33 +675,40 @@ cudaError_t launch(CgArgs a, int warps, cudaStream_t st) {
 }
 
 // Which lanes, warps and CTAs.  Four lanes per node group measured fastest where ten or more warps' copies fit
-// an SM (64^3 Hexa8, FP32 values: 75 us an iteration, 88 with eight lanes; 32^3, FP64 values: 29 against 33);
-// longer rows (Hexa20: 24 against 25 us at 24 x 24 x 12) and per-entry columns take eight.  A system that leaves
-// SMs without work takes four warps per CTA (12^3 Hexa8: 12 us against 16 with sixteen), and one that fits 64
-// warps runs as one cluster of eight CTAs, whose barriers cost a third of the grid's (40 x 8 plate: 7.0 us an
-// iteration against 9.2; at 8^3 Hexa8, 92 warps, the grid is ahead by 15 %).
+// an SM (64^3 Hexa8, FP32 values: 75 us an iteration, 88 with eight lanes; 32^3, FP64 values: 29 against 33); where they
+// do not, eight.  Per-entry columns the same (64^3: 151 against 198 us; the three kernels of before 173), but eight
+// as long as every warp has one chunk at most (10 x 10 x 5 Hexa20: 11 us against 12), and for FP64 values whose number is
+// not known, as the longer rows of Hexa20 would not fit (16 x 16 x 8: 24 us against 30).  A system that leaves SMs
+// without work takes four warps per CTA (12^3 Hexa8: 12 us against 16 with sixteen), and one that fits 64 warps runs as
+// one cluster of eight CTAs, whose barriers cost a third of the grid's (40 x 8 plate: 7.0 us an iteration against
+// 9.2; at 8^3 Hexa8, 92 warps, the grid is ahead by 15 %).
 template <typename KT, bool FF, int PB, int BS>
 cudaError_t dispatch(CgArgs a, int64_t nnz, cudaStream_t st) {
+  constexpr int budget = 227 * 1024 - 14 * 1024;  // shared memory of a CTA less the static arrays
   // a warp's copy: its chunk's entries, 15 % more than on average (longer chunks are read from global memory),
-  // and their column list
+  // and their column list; all that sixteen warps can have if the number of entries is not known
   const int64_t groups = a.n / PB;
-  const double perGroup = nnz > 0 ? (double)nnz / (double)groups : 243.0;
   auto stage = [&](int lpg) {
-    const int64_t entries = std::min<int64_t>((int64_t)(1.15 * perGroup * (32 / lpg)) + 16, 24 * 1024 / (int)sizeof(KT));
+    int64_t entries = budget / MAX_WARPS * (PB * PB) / ((int)sizeof(KT) * PB * PB + 4) - 16;
+    if (nnz > 0)
+      entries = std::min<int64_t>((int64_t)(1.15 * ((double)nnz / (double)groups) * (32 / lpg)) + 16, 24 * 1024 / (int)sizeof(KT));
     a.capK = (int)((entries * (int)sizeof(KT) + 31) / 16 * 16);
     a.capC = (int)((entries / (PB * PB) * 4 + 47) / 16 * 16);
     return a.capK + a.capC;
   };
-  constexpr int budget = 227 * 1024 - 14 * 1024;  // shared memory of a CTA less the static arrays
-  const int lpg = PB == 1 || 10 * stage(4) > budget ? 8 : 4;
+  const bool eight = PB == 1 && ((groups + 3) / 4 <= (int64_t)pcg_sms() * MAX_WARPS || (nnz <= 0 && sizeof(KT) == 8));
+  const int lpg = eight || 10 * stage(4) > budget ? 8 : 4;
   const int64_t chunks = (groups + 32 / lpg - 1) / (32 / lpg);
   const int most = std::min(MAX_WARPS, budget / stage(lpg));
   const bool cluster = chunks <= 64 && most >= 8;
   int warps = (int)std::min<int64_t>(most, std::max<int64_t>(4, (chunks + pcg_sms() - 1) / pcg_sms()));
   if (cluster) warps = (int)std::max<int64_t>(1, (chunks + MAX_CLUSTER - 1) / MAX_CLUSTER);
   warps = std::max(warps, 3);  // a warp for each sum
-  if constexpr (PB > 1) {
-    if (lpg == 4) return cluster ? launch<KT, FF, PB, BS, 4, true>(a, warps, st) : launch<KT, FF, PB, BS, 4, false>(a, warps, st);
+  if (lpg == 4) {
+    if constexpr (PB > 1) {  // per-entry columns: not in a system of 64 warps
+      if (cluster) return launch<KT, FF, PB, BS, 4, true>(a, warps, st);
+    }
+    return launch<KT, FF, PB, BS, 4, false>(a, warps, st);
   }
   return cluster ? launch<KT, FF, PB, BS, 8, true>(a, warps, st) : launch<KT, FF, PB, BS, 8, false>(a, warps, st);
 }
