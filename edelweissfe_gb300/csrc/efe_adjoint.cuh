@@ -17,10 +17,11 @@
 //
 // The sums over the nodes (J, and H and Lambda before their product with J^-T) and the element's nodal sums of
 // dL/dJ dN/dxi run in fixed-point integers (efe_fixed.cuh), H and Lambda also through that product: the FP64 pipe, which
-// binds the kernel, is left with about 380 instructions per point.  Nodal values are staged once per element, relative
+// binds the kernel, is left with about 380 instructions per point.  Each component of the nodal values, of J^-T and of
+// dL/dJ has a scale of its own: in thin elements they differ in size.  Nodal values are staged once per element, relative
 // to its first node (sum_a dN_a = 0), and dN/dxi once per CTA, whose elements are strided by the grid.  Four CTAs per
-// SM (128 registers): 32768 C3D8TL elements in 256 us, about 160 of them the FP64 pipe's, against 486 with float-float
-// sums and products by M; 2048 C3D20TL 148 against 297 us; 20000 CPE8RTL 96 against 150 us.
+// SM (128 registers): 32768 C3D8TL elements in 227 us, about 160 of them the FP64 pipe's, against 486 with float-float
+// sums and products by M; 2048 C3D20TL 122 against 282 us; 20000 CPE8RTL 52 against 108 us.
 #pragma once
 #include "efe_launch.cuh"
 
@@ -57,8 +58,9 @@ struct AdjointTLLayout {
   static constexpr size_t d_off = 0;                          // fx [NQ][DS]: dN/dxi
   static constexpr size_t x_off = d_off + 8 * NQ * DS;        // double, then fx [EPB][XS: X, U, lambda][NN][DIM]
   static constexpr size_t j_off = x_off + 8 * EPB * XS;       // double, then fx [NP][JS]: dL/dJ
-  static constexpr size_t e_off = j_off + 8 * NP * JS;        // int: scales [EPB][X, U, lambda, dL/dJ], [1] dN/dxi
-  static constexpr size_t bytes = e_off + 4 * (4 * EPB + 1);
+  static constexpr int ES = 4 * DIM;                          // scales of an element: components of X, U, lambda, dL/dJ
+  static constexpr size_t e_off = j_off + 8 * NP * JS;        // int [EPB][ES], [1] dN/dxi
+  static constexpr size_t bytes = e_off + 4 * (ES * EPB + 1);
   static_assert(NN <= 31 && NQ <= 31, "products of a fixed-point sum");
 };
 
@@ -95,7 +97,7 @@ template <int SHAPE, int RULE>
 __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
   using L = AdjointTLLayout<SHAPE, RULE>;
   constexpr int DIM = L::DIM, NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NT = L::NT, EPB = L::EPB, DS = L::DS, JS = L::JS,
-                XS = L::XS;
+                XS = L::XS, ES = L::ES;
   extern __shared__ __align__(16) unsigned char smem[];
   fx* sD = reinterpret_cast<fx*>(smem + L::d_off);
   double* sXd = reinterpret_cast<double*>(smem + L::x_off);
@@ -103,7 +105,7 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
   double* sJd = reinterpret_cast<double*>(smem + L::j_off);
   fx* sJ = reinterpret_cast<fx*>(smem + L::j_off);
   int* sem = reinterpret_cast<int*>(smem + L::e_off);
-  int* semD = sem + 4 * EPB;
+  int* semD = sem + ES * EPB;
   const int tid = threadIdx.x;
   const int le = tid / NQ, q = tid - le * NQ;
   double xi, eta, zeta, w;
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
 
   for (int64_t e0 = (int64_t)blockIdx.x * EPB; e0 < ar.nEl; e0 += (int64_t)gridDim.x * EPB) {
     const int nLoc = ar.nEl - e0 < EPB ? (int)(ar.nEl - e0) : EPB;
-    for (int t = tid; t < 4 * EPB; t += NT) sem[t] = 0;
+    for (int t = tid; t < ES * EPB; t += NT) sem[t] = 0;
     __syncthreads();
     // ---- nodal values relative to the element's first node
     for (int t = tid; t < nLoc * NN; t += NT) {
@@ -157,29 +159,26 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
         v[2][c] = ar.lam[dof + c] - ar.lam[dof0 + c];
       }
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        int em = 0;
+      for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int c = 0; c < DIM; ++c) {
-          em = max(em, fx_exponent(v[k][c]));
           sXd[l * XS + k * NDOF + a * DIM + c] = v[k][c];
+          atomicMax(sem + l * ES + k * DIM + c, fx_exponent(v[k][c]));
         }
-        atomicMax(sem + l * 4 + k, em);
-      }
     }
     __syncthreads();
     for (int t = tid; t < nLoc * 3 * NDOF; t += NT) {
       const int l = t / (3 * NDOF), r = t - l * 3 * NDOF;
-      sX[l * XS + r] = fx_make(sXd[l * XS + r], sem[l * 4 + r / NDOF]);
+      sX[l * XS + r] = fx_make(sXd[l * XS + r], sem[l * ES + r / NDOF * DIM + r % DIM]);
     }
     __syncthreads();
 
     // ---- a thread per point
     const int64_t e = e0 + le;
     const bool live = le < nLoc;
-    int ej = 0;
     if (live) {
       const int emD = *semD;
+      int* el = sem + le * ES;
       // sum_a v_a[c] D[r][a] as integers, V[c][r]
       auto nodal = [&](int k, int row2, FxSum V[DIM][DIM]) {
 #pragma unroll
@@ -207,7 +206,7 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
 #pragma unroll
         for (int c = 0; c < DIM; ++c)
 #pragma unroll
-          for (int r = 0; r < DIM; ++r) J[r][c] = fx_value(fx_int(V[c][r]), emD + sem[le * 4]);
+          for (int r = 0; r < DIM; ++r) J[r][c] = fx_value(fx_int(V[c][r]), emD + el[c]);
       }
       if constexpr (SHAPE == EFE_HEXA20) {
         const int64_t n0 = ar.conn[e * NN];
@@ -218,24 +217,24 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
       // H and Lambda: the nodal sums times J^-T
       double F[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, H[DIM][DIM], Lam[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
       {
-        int ei = 0;
-#pragma unroll
-        for (int c = 0; c < DIM; ++c)
-#pragma unroll
-          for (int r = 0; r < DIM; ++r) ei = max(ei, fx_exponent(iJ[c][r]));
+        int ei[DIM];
         fx iJf[DIM][DIM];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c)
+        for (int c = 0; c < DIM; ++c) {
+          ei[c] = 0;
 #pragma unroll
-          for (int r = 0; r < DIM; ++r) iJf[c][r] = fx_make(iJ[c][r], ei);
+          for (int r = 0; r < DIM; ++r) ei[c] = max(ei[c], fx_exponent(iJ[c][r]));
+#pragma unroll
+          for (int r = 0; r < DIM; ++r) iJf[c][r] = fx_make(iJ[c][r], ei[c]);
+        }
         constexpr int B = NN > 8 ? 5 : (NN > 4 ? 4 : 3);  // |sum| <= NN 2^58 as an operand of 57 bits
 #pragma unroll
         for (int k = 1; k < 3; ++k) {
           FxSum V[DIM][DIM];
           nodal(k, 2, V);
-          const int em = emD + sem[le * 4 + k] - 1023 + B;  // the operand's scale: its value is V 2^(em - 1079)
 #pragma unroll
           for (int i = 0; i < DIM; ++i) {
+            const int em = emD + el[k * DIM + i] - 1023 + B;  // the operand's scale: its value is V 2^(em - 1079)
             fx v[DIM];
 #pragma unroll
             for (int r = 0; r < DIM; ++r) v[r] = fx_split(fx_int(V[i][r], -B));
@@ -244,7 +243,7 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
               FxSum t{0, 0};
 #pragma unroll
               for (int r = 0; r < DIM; ++r) fx_fma(t, v[r], iJf[j][r]);
-              const double x = fx_value(fx_int(t), em + ei);
+              const double x = fx_value(fx_int(t), em + ei[j]);
               if (k == 1) {
                 H[i][j] = x;
                 F[i][j] += x;
@@ -305,9 +304,10 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
         }
       }
 #pragma unroll
-      for (int r = 0; r < DIM; ++r)
+      for (int c = 0; c < DIM; ++c) {
+        int ej = 0;
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) {
+        for (int r = 0; r < DIM; ++r) {
           double v = 0.0;
 #pragma unroll
           for (int k = 0; k < DIM; ++k) v = fma(iJ[k][r], E[k][c], v);
@@ -315,12 +315,13 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
           sJd[tid * JS + r * DIM + c] = v;
           ej = max(ej, fx_exponent(v));
         }
-      atomicMax(sem + le * 4 + 3, ej);
+        atomicMax(el + 3 * DIM + c, ej);
+      }
     }
     __syncthreads();
     if (live) {
 #pragma unroll
-      for (int k = 0; k < DIM * DIM; ++k) sJ[tid * JS + k] = fx_make(sJd[tid * JS + k], sem[le * 4 + 3]);
+      for (int k = 0; k < DIM * DIM; ++k) sJ[tid * JS + k] = fx_make(sJd[tid * JS + k], sem[le * ES + 3 * DIM + k % DIM]);
     }
     __syncthreads();
     // ---- the element's nodal sums: gX[a][c] += sum_q sum_r dL/dJ[r][c] D[r][a]
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(128, 4) adjoint_tl_kernel(AdjointArgs ar) {
       int64_t v = 0;
 #pragma unroll
       for (int r = 0; r < DIM; ++r) v += fx_int(acc[r], -2);
-      atomicAdd(ar.gX + (int64_t)ar.conn[(e0 + l) * NN + a] * DIM + c, fx_value(v, *semD + sem[l * 4 + 3] + 2));
+      atomicAdd(ar.gX + (int64_t)ar.conn[(e0 + l) * NN + a] * DIM + c, fx_value(v, *semD + sem[l * ES + 3 * DIM + c] + 2));
     }
     __syncthreads();
   }

@@ -26,9 +26,9 @@
 // adjoints (plain stores: one thread owns an element's property).
 //
 // Measured, before (FP64 or float-float sums, the coordinate adjoint node by node and point by point) and now: C3D20,
-// 6912 elements 218 -> 211 us (the reverse return map keeps the FP64 pipe half busy with eleven warps per SM, which
-// shared memory bounds); C3D20 fp64, 1728 elements 110 -> 65 us, with gX 319 -> 189; C3D8, 32768 elements 208 -> 190 us, with
-// gX 518 -> 350.
+// 6912 elements 219 -> 201 us (the reverse return map keeps the FP64 pipe half busy with eleven warps per SM, which
+// shared memory bounds); C3D20 fp64, 1728 elements 111 -> 63 us, with gX 319 -> 201; C3D8, 32768 elements 208 -> 188 us, with
+// gX 518 -> 316.
 #pragma once
 #include "efe_launch.cuh"
 
@@ -369,8 +369,8 @@ struct SSAdjointTile {
   static constexpr int DIM = ShapeInfo<SHAPE>::DIM, NN = ShapeInfo<SHAPE>::NN, NQ = RuleInfo<RULE>::NQ;
   static constexpr int NDOF = NN * DIM, NT = 128;
   // per element: dU_e and PBar_e; its points' dN/dX (NDOF x NQ, 8 bytes each: doubles, then digits), property adjoints
-  // (6) and strain adjoints (6)
-  static constexpr size_t per_el = sizeof(double) * (2 * NDOF + NQ * NDOF + NQ * 12);
+  // (6) and strain adjoints (a factor for each row and direction)
+  static constexpr size_t per_el = sizeof(double) * (2 * NDOF + NQ * NDOF + NQ * (6 + DIM * DIM));
   static constexpr int EPB0 = NT / NQ > 0 ? NT / NQ : 1;
   static constexpr int EPB = (size_t)EPB0 * per_el <= 96 * 1024 ? EPB0 : (int)((96 * 1024) / per_el);
   static_assert(EPB >= 1, "one element must fit in shared memory");
@@ -382,13 +382,16 @@ struct SSAdjointTile {
   static constexpr size_t u_off = 0, p_off = u_off + sizeof(double) * EPB * NDOF,
                           g_off = up_bytes > qq_bytes ? up_bytes : qq_bytes,
                           q_off = g_off + sizeof(double) * NDOF * NPS,  // double [NP][6]: property adjoints
-                          d_off = q_off + sizeof(double) * NP * 6,      // fx [NP][6]: strain adjoints
-                          c_off = d_off + sizeof(double) * NP * 6,      // SSRevConst [EPB]
+                          d_off = q_off + sizeof(double) * NP * 6,      // fx [NP][DIM][DIM]: strain adjoints
+                          c_off = d_off + sizeof(double) * NP * DIM * DIM,  // SSRevConst [EPB]
                           w_off = c_off + sizeof(SSRevConst) * EPB,     // double [NP][3]: W
                           e_off = w_off + (GX && SHAPE == EFE_HEXA20 ? sizeof(double) * NP * 3 : 0),
-                          bytes = e_off + sizeof(int) * 4 * EPB;  // int [EPB][4]: scales of dU, PBar, B^T deBar, Q
+                          bytes = e_off + sizeof(int) * 5 * DIM * EPB;
+  // int [EPB][5][DIM]: scales of the components of dU, PBar and dN/dX, of the rows of B^T deBar and of the coordinate
+  // adjoint (as in efe_ss3.cuh: a point's dN/dX has the element's, shifted by t)
+  static constexpr int ES = 5 * DIM, eU = 0, eP = DIM, eD = 2 * DIM, eE = 3 * DIM, eQ = 4 * DIM;
   static_assert(NP <= NT, "a thread per point");
-  static_assert(2 * ((NN + 1) / 2) <= 31 && NQ <= 31, "products of a fixed-point sum");
+  static_assert(NN <= 31 && NQ <= 31, "products of a fixed-point sum");
 };
 
 // The three B-products (B dU, B PBar, B^T deBar) run in fixed-point integers (efe_fixed.cuh) on digits of dN/dX, of the
@@ -400,7 +403,7 @@ struct SSAdjointTile {
 template <int SHAPE, int RULE, bool GX>
 __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss_kernel(SSAdjointArgs a) {
   using T = SSAdjointTile<SHAPE, RULE, GX>;
-  constexpr int DIM = T::DIM, NN = T::NN, NQ = T::NQ, NDOF = T::NDOF, EPB = T::EPB, NT = T::NT, NPS = T::NPS;
+  constexpr int DIM = T::DIM, NN = T::NN, NQ = T::NQ, NDOF = T::NDOF, EPB = T::EPB, NT = T::NT, NPS = T::NPS, ES = T::ES;
   extern __shared__ __align__(128) unsigned char smem[];
   fx* su = reinterpret_cast<fx*>(smem + T::u_off);
   fx* sp = reinterpret_cast<fx*>(smem + T::p_off);
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
 #pragma unroll 10
     for (int r = 0; r < NDOF; ++r) cp_async8(sGd + r * NPS + pl, gp + (int64_t)r * stride);
   }
-  for (int t = threadIdx.x; t < 4 * EPB; t += NT) sem[t] = 0;
+  for (int t = threadIdx.x; t < ES * EPB; t += NT) sem[t] = 0;
   __syncthreads();
   if (NT - 1 - (int)threadIdx.x < nLoc) {
     const int le = NT - 1 - threadIdx.x;
@@ -436,29 +439,41 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
     const int le = t / NN, n = t - le * NN;
     const int32_t* en = a.conn + (e0 + le) * NN;
     const int32_t dof = a.nodeDof[en[n]], dof0 = a.nodeDof[en[0]];
-    int eu = 0, ep = 0;
     for (int c = 0; c < DIM; ++c) {
       const double u = a.dU[dof + c] - a.dU[dof0 + c], p = a.Pbar ? a.Pbar[dof + c] - a.Pbar[dof0 + c] : 0.0;
       sud[le * NDOF + n * DIM + c] = u;
       sud[EPB * NDOF + le * NDOF + n * DIM + c] = p;
-      eu = fx_max_exponent(eu, u);
-      ep = fx_max_exponent(ep, p);
+      atomicMax(sem + le * ES + T::eU + c, fx_exponent(u));
+      atomicMax(sem + le * ES + T::eP + c, fx_exponent(p));
     }
-    atomicMax(sem + le * 4, eu);
-    atomicMax(sem + le * 4 + 1, ep);
   }
   cp_async_wait_all();
+  // the thread's own copies have landed: its point's largest components
+  int eg[DIM] = {};
+  if (live) {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+#pragma unroll 10
+      for (int n = 0; n < NN; ++n) eg[c] = fx_max_exponent(eg[c], sGd[(c * NN + n) * NPS + pl]);
+      atomicMax(sem + pl / NQ * ES + T::eD + c, eg[c]);
+    }
+  }
   __syncthreads();
   for (int t = threadIdx.x; t < 2 * nLoc * NDOF; t += NT) {
     const int w = t >= nLoc * NDOF, k = t - w * nLoc * NDOF;
-    su[w * EPB * NDOF + k] = fx_make(sud[w * EPB * NDOF + k], sem[k / NDOF * 4 + w]);
+    su[w * EPB * NDOF + k] = fx_make(sud[w * EPB * NDOF + k], sem[k / NDOF * ES + w * DIM + k % DIM]);
   }
-  int eg = 0;
   if (live) {
-#pragma unroll 10
-    for (int r = 0; r < NDOF; ++r) eg = fx_max_exponent(eg, sGd[r * NPS + pl]);
+    const int* D = sem + pl / NQ * ES + T::eD;
+    int t = eg[0] - D[0];
+#pragma unroll
+    for (int c = 1; c < DIM; ++c) t = max(t, eg[c] - D[c]);
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      eg[c] = D[c] + t;
 #pragma unroll 4
-    for (int r = 0; r < NDOF; ++r) sG[r * NPS + pl] = fx_make(sGd[r * NPS + pl], eg);
+      for (int n = 0; n < NN; ++n) sG[(c * NN + n) * NPS + pl] = fx_make(sGd[(c * NN + n) * NPS + pl], eg[c]);
+    }
   }
   __syncthreads();
 
@@ -468,38 +483,9 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
     const int le = pl / NQ, q = pl - le * NQ;
     const int64_t e = e0 + le, pt = e0 * NQ + pl;
     const double s = a.geomS[pt];
-    // B u and B PBar (small-strain Voigt 11,22,33,12,13,23, engineering shear)
-    // at most 20 products to a sum: half of the nodes at a time beyond eight
-    constexpr int PARTS = NN > 8 ? 2 : 1;
-    auto strain = [&](const fx* v, int em, double out[6]) {
-      int64_t sum[6] = {0, 0, 0, 0, 0, 0};
-      for (int part = 0; part < PARTS; ++part) {
-        FxSum f[6] = {};
-#pragma unroll 2
-        for (int n = part * (NN / PARTS); n < (part + 1) * (NN / PARTS); ++n) {
-          const fx gx = sG[n * NPS + pl], gy = sG[(NN + n) * NPS + pl];
-          const fx vx = v[n * DIM], vy = v[n * DIM + 1];
-          fx_fma(f[0], gx, vx);
-          fx_fma(f[1], gy, vy);
-          fx_fma(f[3], gy, vx);
-          fx_fma(f[3], gx, vy);
-          if constexpr (DIM == 3) {
-            const fx gz = sG[(2 * NN + n) * NPS + pl], vz = v[n * DIM + 2];
-            fx_fma(f[2], gz, vz);
-            fx_fma(f[4], gz, vx);
-            fx_fma(f[4], gx, vz);
-            fx_fma(f[5], gz, vy);
-            fx_fma(f[5], gy, vz);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) sum[k] += fx_int(f[k], 1 - PARTS);
-      }
-#pragma unroll
-      for (int k = 0; k < 6; ++k) out[k] = fx_value(sum[k], em + eg + PARTS - 1);
-    };
-    // the gradient as well: out from its symmetric part, summed in integers
-    auto gradient = [&](const fx* v, int em, double out[6], double H[DIM][DIM]) {
+    // B u and B PBar (small-strain Voigt 11,22,33,12,13,23, engineering shear) from the gradient sums (l, c): component l of
+    // the values, direction c of dN/dX; with H, the gradient too
+    auto strain = [&](const fx* v, const int* em, double out[6], double H[DIM][DIM]) {
       FxSum f[DIM][DIM] = {};
 #pragma unroll 2
       for (int n = 0; n < NN; ++n) {
@@ -513,17 +499,22 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
           for (int c = 0; c < DIM; ++c) fx_fma(f[l][c], x, g[c]);
         }
       }
-      int64_t I[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+      for (int k = 0; k < 6; ++k) out[k] = 0.0;
 #pragma unroll
       for (int l = 0; l < DIM; ++l)
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) {
-          I[l][c] = fx_int(f[l][c], -1);
-          H[l][c] = fx_value(I[l][c], em + eg + 1);
+        for (int c = l; c < DIM; ++c) {
+          int sc = em[l] + eg[c];
+          int64_t I = fx_int(f[l][c], -1);
+          if constexpr (GX) H[l][c] = fx_value(I, sc + 1);
+          if (l != c) {
+            const int64_t K = fx_int(f[c][l], -1);
+            if constexpr (GX) H[c][l] = fx_value(K, em[c] + eg[l] + 1);
+            I = fx_add(I, sc, K, em[c] + eg[l]);
+          }
+          out[l == c ? l : l + c + 2] = fx_value(I, sc + 1);
         }
-      const int64_t sum[6] = {I[0][0], I[1][1], I[2][2], I[0][1] + I[1][0], I[0][2] + I[2][0], I[1][2] + I[2][1]};
-#pragma unroll
-      for (int k = 0; k < 6; ++k) out[k] = fx_value(sum[k], em + eg + 1);
     };
     // seeds and the state before the increment, loaded ahead of the sums
     double sBar[6], eBar[6], kBar = 0.0, sig0[6], k0 = 0.0;
@@ -537,13 +528,8 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
     if (vm) k0 = a.stateBefore[(int64_t)12 * stride + pt];
     double de[6], bp[6];
     double Hu[DIM][DIM], Hp[DIM][DIM];
-    if constexpr (GX) {
-      gradient(su + le * NDOF, sem[le * 4], de, Hu);
-      gradient(sp + le * NDOF, sem[le * 4 + 1], bp, Hp);
-    } else {
-      strain(su + le * NDOF, sem[le * 4], de);
-      strain(sp + le * NDOF, sem[le * 4 + 1], bp);
-    }
+    strain(su + le * NDOF, sem + le * ES + T::eU, de, Hu);
+    strain(sp + le * NDOF, sem + le * ES + T::eP, bp, Hp);
     // P_e = -sum_q s B^T sig  =>  sigBar -= s B PBar
 #pragma unroll
     for (int f = 0; f < 6; ++f) sBar[f] -= s * bp[f];
@@ -585,25 +571,34 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
     if constexpr (GX) {
       double W[3] = {0.0, 0.0, 0.0};
       coordinate_adjoint<SHAPE, RULE, DIM>(a, e, q, s, mc, vm, planeStress, sig0, k0, de, deBar, bp, Hu, Hp, Q, W);
-      int eq = 0;
 #pragma unroll
-      for (int k = 0; k < DIM; ++k)
+      for (int c = 0; c < DIM; ++c) {
+        int eq = 0;
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) eq = fx_max_exponent(eq, Q[k][c]);
-      atomicMax(sem + le * 4 + 3, eq + eg);
+        for (int k = 0; k < DIM; ++k) eq = max(eq, fx_exponent(Q[k][c]) + eg[k]);
+        atomicMax(sem + le * ES + T::eQ + c, eq);
+      }
       if constexpr (SHAPE == EFE_HEXA20)
         for (int c = 0; c < 3; ++c) sW[pl * 3 + c] = W[c];
     }
-    int ed = 0;
-    for (int f = 0; f < 6; ++f) ed = fx_max_exponent(ed, deBar[f]);
-    atomicMax(sem + le * 4 + 2, ed + eg);
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      int ed = 0;
+#pragma unroll
+      for (int l = 0; l < DIM; ++l) ed = max(ed, fx_exponent(deBar[l == c ? c : l + c + 2]) + eg[l]);
+      atomicMax(sem + le * ES + T::eE + c, ed);
+    }
   }
   __syncthreads();
   if (live) {
-    for (int f = 0; f < 6; ++f) sd[pl * 6 + f] = fx_make(deBar[f], sem[pl / NQ * 4 + 2] - eg);
-    if constexpr (GX)
-      for (int k = 0; k < DIM; ++k)
-        for (int c = 0; c < DIM; ++c) sQ[(pl * DIM + k) * DIM + c] = fx_make(Q[k][c], sem[pl / NQ * 4 + 3] - eg);
+    const int* el = sem + pl / NQ * ES;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+#pragma unroll
+      for (int l = 0; l < DIM; ++l) {
+        sd[(pl * DIM + c) * DIM + l] = fx_make(deBar[l == c ? c : l + c + 2], el[T::eE + c] - eg[l]);
+        if constexpr (GX) sQ[(pl * DIM + l) * DIM + c] = fx_make(Q[l][c], el[T::eQ + c] - eg[l]);
+      }
   }
   __syncthreads();
 
@@ -613,17 +608,15 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
   for (int t = threadIdx.x; t < nLoc * NDOF; t += NT) {
     const int le = t / NDOF, k = t - le * NDOF, n = k / DIM, c = k - n * DIM;
     const int64_t e = e0 + le;
-    // row c: 3D (11 12 13 | 12 22 23 | 13 23 33) = Voigt (0 3 4 | 3 1 5 | 4 5 2); 2D (0 3 | 3 1)
-    const int v0 = c == 0 ? 0 : (c == 1 ? 3 : 4), v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
     FxSum f[3] = {};  // one for each direction
 #pragma unroll 3
     for (int q = 0; q < NQ; ++q) {
       const int p = le * NQ + q;
-      fx_fma(f[0], sd[p * 6 + v0], sG[n * NPS + p]);
-      fx_fma(f[1], sd[p * 6 + v1], sG[(NN + n) * NPS + p]);
-      if constexpr (DIM == 3) fx_fma(f[2], sd[p * 6 + v2], sG[(2 * NN + n) * NPS + p]);
+      const fx* row = sd + (p * DIM + c) * DIM;
+#pragma unroll
+      for (int l = 0; l < DIM; ++l) fx_fma(f[l], row[l], sG[(l * NN + n) * NPS + p]);
     }
-    const double v = fx_value(fx_int(f[0], -2) + fx_int(f[1], -2) + fx_int(f[2], -2), sem[le * 4 + 2] + 2);
+    const double v = fx_value(fx_int(f[0], -2) + fx_int(f[1], -2) + fx_int(f[2], -2), sem[le * ES + T::eE + c] + 2);
     const int32_t node = a.conn[e * NN + n];
     atomicAdd(a.dUbar + a.nodeDof[node] + c, v);
     if constexpr (GX) {
@@ -634,7 +627,7 @@ __global__ void __launch_bounds__(SSAdjointTile<SHAPE, RULE, GX>::NT) adjoint_ss
 #pragma unroll
         for (int l = 0; l < DIM; ++l) fx_fma(h[l], sQ[(p * DIM + l) * DIM + c], sG[(l * NN + n) * NPS + p]);
       }
-      double x = fx_value(fx_int(h[0], -2) + fx_int(h[1], -2) + fx_int(h[2], -2), sem[le * 4 + 3] + 2);
+      double x = fx_value(fx_int(h[0], -2) + fx_int(h[1], -2) + fx_int(h[2], -2), sem[le * ES + T::eQ + c] + 2);
       if constexpr (SHAPE == EFE_HEXA20) {
         double w = 0.0;
         for (int q = 0; q < NQ; ++q) w += sW[(le * NQ + q) * 3 + c];

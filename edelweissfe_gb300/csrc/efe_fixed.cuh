@@ -6,8 +6,11 @@
 // |l| <= 2^27, and a product costs three multiply-adds into two accumulators (h h, and h l + l h together; l l, below
 // 2^-60 of the largest product, is left out): 18 products per clock and SM, ten times the FP64 pipe.  The accumulation
 // is exact; what is lost is the rounding of the operands to the common scale, 2^-58 of the largest operand (FP64
-// rounds every product and sum at 2^-53).  At most 31 products to a sum (h h reaches 2^58).  em: biased exponent of the
-// largest operand.  Scales are integers that may leave the exponent range; FX_NAN marks non-finite operands.
+// rounds every product and sum at 2^-53).  The error is thus one of the largest operands' product, not of the sum's own
+// terms: operands share a scale only where they are of one size by their nature, in an element the values of one component.
+// The components of dN/dX of a thin element, and of the displacements of a plate, are not, and have scales of their own.
+// At most 31 products to a sum (h h reaches 2^58).  em: biased exponent of the largest operand.  Scales are integers
+// that may leave the exponent range; FX_NAN marks non-finite operands.
 #pragma once
 #include <cstdint>
 
@@ -53,6 +56,22 @@ __device__ __forceinline__ int64_t fx_int(const FxSum& s, int B = 0) {
   if (B < 0) return fx_shift(s.hh + (s.cr >> 28), -B);
   return (s.hh << B) + (B < 28 ? (s.cr + (1ll << 27 >> B)) >> (28 - B) : 0);
 }
+// V / 2^d rounded down, for sums that keep bits to spare: one unit is 2^-57 or less of what they can hold
+__device__ __forceinline__ int64_t fx_down(int64_t V, int d) { return V >> min(d, 63); }
+// A + B of scales sa, sb (fx_int of both with B = -1, so that the sum fits); sa becomes the sum's scale, less that shift
+__device__ __forceinline__ int64_t fx_add(int64_t A, int& sa, int64_t B, int sb) {
+  const int m = max(sa, sb);
+  const int64_t v = fx_down(A, m - sa) + fx_down(B, m - sb);
+  sa = m;
+  return v;
+}
+// An operand of scale em as a float, from its upper digit: unit = fx_unit(em)
+__device__ __forceinline__ float fx_unit(int em) {
+  const int e = em - 1051 + 127;
+  if (e > 0 && e < 255) return __int_as_float(e << 23);
+  return em >= FX_NAN ? __int_as_float(0x7fc00000) : ldexpf(1.0f, max(-300, min(300, em - 1051)));
+}
+__device__ __forceinline__ float fx_float(fx v, float unit) { return (float)v.h * unit; }
 // the upper 32 bits of |hh|, roughly: __clz of them (or of an OR of several) counts the places to spare
 __device__ __forceinline__ int fx_bits(const FxSum& s) {
   const int h = (int)(s.hh >> 32);

@@ -31,8 +31,8 @@ struct TileOf {
                               : (bytes <= 72 * 1024 ? 3 : 1);
 };
 // The warp tile of small-strain Hexa8 with an FP32 tangent (efe_ss3.cuh), one shape for all variants: six CTAs of
-// four warps per SM hold the kernel to 80 registers (40 B of spills); five CTAs (96 registers) or four (128) run in 1.01
-// and 1.06 times its time on 262144 elements, 1.00 and 1.05 times on 65231.
+// four warps per SM hold the kernel to 80 registers (48 B of spills); five CTAs (96 registers) or four (128) run in 1.00
+// and 1.04 times its time on 262144 elements, 1.02 and 1.05 times on 65231.
 template <int VARIANT>
 struct WarpTile {
   static constexpr int NT = VARIANT == SMALL_TILE ? 32 : 128, EPB = SS3Hexa8Layout<NT>::EPB, MINB = VARIANT == SMALL_TILE ? 1 : 6;
@@ -40,7 +40,7 @@ struct WarpTile {
 };
 // The two-element tile of Hexa20 3x3x3 with an FP32 tangent (efe_ss3.cuh), one shape for all variants, the number 3 of the
 // former tensor-core tile among them: five CTAs per SM (96 registers).  Small strain, 13824 elements: four (128 registers)
-// or six (80, 116 B of spills) run in 1.06 and 1.07 times its time; total Lagrangian, 2730 elements: four in 1.14.
+// or six (80) run in 1.03 and 1.17 times its time; total Lagrangian, 2730 elements: four in 1.16, six in 1.03.
 template <bool TL>
 struct Hexa20Tile {
   static constexpr int NT = Hexa20Layout<TL>::NT, EPB = Hexa20Layout<TL>::EPB, MINB = 5;

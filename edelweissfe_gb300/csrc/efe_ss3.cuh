@@ -8,15 +8,20 @@
 // over few terms of one scale per element, so they run as integer multiply-adds and are exact apart from the
 // rounding of the operands.
 //
-// Scales (biased exponents): dN/dX of a point em_g, the element's dU em_u, over the element's points of s sigma
-// times the point's dN/dX em_s, of the tangent's coefficients (c12 s and c44 s; a s) times dN/dX twice em_c, em_a: the
-// per-point factors are rounded relative to em_s - em_g, em_c - 2 em_g and em_a - 2 em_g, so that all points of a sum
-// share one scale.
+// Scales (biased exponents), one per component, as the components of dN/dX (thin elements) and of the increment
+// (plates, rotations) differ in size by their nature: component d of the element's dN/dX has D_d, a point the same shift
+// t <= 0 of all three (its dN/dX is smaller), so that D_d + t holds it; component c of dU has U_c.  A normal strain is one
+// sum, a shear two, of the scales D_j + U_i and D_i + U_j.  A row c of the residual has E_c, the largest s sigma_cd times
+// dN/dX_d of the element: the point's factors are rounded relative to E_c - D_d - t, nine instead of six.  The FP64 tangent's
+// coefficients (c12 s and c44 s; a s) have em_c and em_a over the points' c 2^2t; its sums (j, k) then em_c + D_j + D_k, the
+// flow direction's em_a + Z_j + Z_k with Z_j the largest n_jd dN/dX_d.
 //
-// Measured, von Mises plastic increment, kernel time before (FP64 sums) and with integers: C3D8, FP64 tangent, 31713
-// elements 1027 -> 362 us; FP32 tangent, 262144 elements 1318 -> 995 us; C3D20, FP64 tangent, 2448 elements 1638 -> 325
-// us; FP32 tangent, 13824 elements 678 -> 380 us.  Largest error against 80-bit arithmetic, before and now: C3D8 P 2.5e-15
-// -> 2.2e-15, K 7.2e-16 -> 7.1e-16; C3D20 P 5.4e-15 -> 5.3e-15, K 1.89e-15 -> 1.88e-15; FP32 K 6.1e-8 in both.
+// Measured, von Mises plastic increment, kernel time before (FP64 sums) and with integers: C3D8, FP64 tangent, 29667
+// elements 1027 -> 346 us; FP32 tangent, 262144 elements 1322 -> 992 us; C3D20, FP64 tangent, 2448 elements 1640 -> 321
+// us; FP32 tangent, 13824 elements 675 -> 383 us (with one scale for all components 363, 985, 326 and 381).  Norm of the
+// error against 113-bit arithmetic, before and now: C3D8, 12 x 11 x 10, P 1.11e-15 -> 1.01e-15, K 4.66e-16 -> 4.62e-16,
+// stress 7.4e-16 -> 5.0e-16; C3D20, 9 x 8 x 5, P 3.10e-15 -> 2.97e-15, K 1.31e-15 -> 1.29e-15; FP32 K of C3D8 6.35e-8 ->
+// 6.23e-8.  In plates of 1 : 10^5 every strain is within the rounding of its own FP64 sum.
 //
 // FP64 tangent: K_ab = sum_q  c12 s G_a (x) G_b + c44 s (G_b (x) G_a + G_a . G_b I) - a s nG_a (x) nG_b.  The
 // operands c12 s G, c44 s G, -a s nG and nG of every point and node are formed once (integer products of the
@@ -30,7 +35,7 @@ struct SS3Layout {
   static constexpr int DIM = 3, NN = ShapeInfo<SHAPE>::NN, NQ = RuleInfo<RULE>::NQ, NDOF = 3 * NN, NP = EPB * NQ;
   static constexpr bool F64 = std::is_same<KT, double>::value;
   // odd strides per point: consecutive points fall on different banks
-  static constexpr int GS = NDOF | 1, SV = (2 * NDOF) | 1, DS = 7;
+  static constexpr int GS = NDOF | 1, SV = (2 * NDOF) | 1, DS = 9;
   static constexpr size_t u_off = 0;                                         // double, then fx [EPB][NDOF]
   static constexpr size_t g_off = u_off + 8 * EPB * NDOF;                    // fx [NP][GS]: dN/dX
   static constexpr size_t d_off = g_off + 8 * NP * GS;                       // [NP][DS]: strain, then s sigma (double, fx)
@@ -40,16 +45,29 @@ struct SS3Layout {
   static constexpr size_t c_off = (n_off + (F64 || NN > 8 || NQ > 8 ? sizeof(KT) * NP * DS : 0) + 7) / 8 * 8;  // KT [NP][3]: coefficients
   static constexpr size_t mc_off = (c_off + sizeof(KT) * NP * 3 + 15) / 16 * 16;  // VMConst [EPB]
   static constexpr size_t rl_off = mc_off + sizeof(VMConst) * EPB;                // int [EPB][NN]
-  static constexpr size_t e_off = rl_off + sizeof(int) * EPB * NN;                // int [EPB]: em_u, em_s, em_c, em_a; [NP]: em_g
-  static constexpr size_t bytes = e_off + sizeof(int) * (4 * EPB + NP);
+  static constexpr int ES = 14;                                                   // scales of an element: U, D, E, Z, em_c, em_a
+  static constexpr size_t e_off = rl_off + sizeof(int) * EPB * NN;                // int [EPB][ES]; [NP][3]: a point's maxima; [NP]: t
+  static constexpr size_t bytes = e_off + sizeof(int) * (ES * EPB + 4 * NP);
 };
 
 __device__ __forceinline__ int fx_max_exponent(int em, double x) { return max(em, fx_exponent(x)); }
 
+// Where the factors of a point's rows lie: digit of (row c, direction d), from the Voigt value of the same place; a shear
+// value has one for each of its rows.
+__device__ __forceinline__ constexpr int row_slot(int c, int d) {
+  return c == 0 ? (d == 0 ? 0 : 2 + d) : c == 1 ? (d == 0 ? 6 : d == 1 ? 1 : 5) : (d == 2 ? 2 : 7 + d);
+}
+// The digits of Voigt value f of a point in its row's scale: E[c] - D[d] - t, with E and D the element's.
+__device__ __forceinline__ void row_digits(fx* out, double x, int f, const int* E, const int* D, int t) {
+  const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+  if (f >= 3) out[f + 3] = fx_make(x, E[j] - D[i] - t);
+  out[f] = fx_make(x, E[i] - D[j] - t);
+}
+
 template <int SHAPE, int RULE, typename KT, int EPB, int NT>
 __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int64_t e0, unsigned char* smem) {
   using L = SS3Layout<SHAPE, RULE, KT, EPB>;
-  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, GS = L::GS, SV = L::SV, DS = L::DS;
+  constexpr int NN = L::NN, NQ = L::NQ, NDOF = L::NDOF, NP = L::NP, GS = L::GS, SV = L::SV, DS = L::DS, ES = L::ES;
   constexpr bool F64 = L::F64;
   // one thread forms a point's digits and strain where a point has few nodes (the tile has a thread per point)
   constexpr bool PERPOINT = NN == 8 && NP <= NT;
@@ -66,16 +84,20 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
   fx* scf = reinterpret_cast<fx*>(smem + L::c_off);
   VMConst* smc = reinterpret_cast<VMConst*>(smem + L::mc_off);
   int* srl = reinterpret_cast<int*>(smem + L::rl_off);
-  int* emu = reinterpret_cast<int*>(smem + L::e_off);
-  int *ems = emu + EPB, *emc = ems + EPB, *ema = emc + EPB, *emg = ema + EPB;
+  int* sem = reinterpret_cast<int*>(smem + L::e_off);
+  constexpr int eU = 0, eD = 3, eE = 6, eZ = 9, eC = 12, eA = 13;  // of an element's ES
+  int *semp = sem + ES * EPB, *semt = semp + 3 * NP;
   const int tid = threadIdx.x;
   const int64_t nEl = g.nElements, stride = nEl * NQ;
   const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB, np = nLoc * NQ;
+  // the shift of a point whose components have the exponents e
+  auto shift = [&](const int* e, const int* el) { return max(max(e[0] - el[eD], e[1] - el[eD + 1]), e[2] - el[eD + 2]); };
 
   // ---- dU relative to the element's first node (sum_a dN_a/dX = 0), row lengths, material constants, dN/dX
-  for (int t = tid; t < 4 * EPB + NP; t += NT) emu[t] = 0;
+  for (int t = tid; t < ES * EPB + 3 * NP; t += NT) sem[t] = 0;
   if (!PERPOINT) __syncthreads();
   double G[PERPOINT ? 3 : 1][PERPOINT ? NN : 1];
+  int eg[3] = {0, 0, 0};
   if constexpr (PERPOINT) {
     if (tid < np) {
 #pragma unroll
@@ -86,10 +108,9 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
   } else {
     for (int t = tid; t < np * NN; t += NT) {
       const int a = t / np, r = t - a * np;
-      int em = 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) em = fx_max_exponent(em, g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + r]);
-      atomicMax(emg + r, em);
+      for (int c = 0; c < 3; ++c)
+        atomicMax(semp + r * 3 + c, fx_exponent(g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + r]));
     }
   }
   for (int t = tid; t < nLoc * NN; t += NT) {
@@ -109,38 +130,48 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
   for (int le = NT - 1 - tid; le < nLoc; le += NT)
     smc[le] = vm_const<!F64>(g.props + (e0 + le) * g.nProps, g.material == EFE_MAT_VON_MISES);
   __syncthreads();
-  for (int t = tid; t < nLoc * NDOF; t += NT) atomicMax(emu + t / NDOF, fx_exponent(su[t]));
-  int eg = 0;
+  for (int t = tid; t < nLoc * NDOF; t += NT) atomicMax(sem + t / NDOF * ES + eU + t % 3, fx_exponent(su[t]));
   if constexpr (PERPOINT) {
     if (tid < np) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
+      for (int c = 0; c < 3; ++c) {
 #pragma unroll
-        for (int a = 0; a < NN; ++a) eg = fx_max_exponent(eg, G[c][a]);
-      emg[tid] = eg;
+        for (int a = 0; a < NN; ++a) eg[c] = fx_max_exponent(eg[c], G[c][a]);
+        atomicMax(sem + tid / NQ * ES + eD + c, eg[c]);
+      }
     }
+  } else {
+    for (int t = tid; t < np * 3; t += NT) atomicMax(sem + t / (3 * NQ) * ES + eD + t % 3, semp[t]);
   }
   __syncthreads();
 
   // ---- digits of dU and dN/dX; the FP32 tangent's dN/dX
-  for (int t = tid; t < nLoc * NDOF; t += NT) suf[t] = fx_make(su[t], emu[t / NDOF]);
+  for (int t = tid; t < nLoc * NDOF; t += NT) suf[t] = fx_make(su[t], sem[t / NDOF * ES + eU + t % 3]);
   if constexpr (PERPOINT) {
     if (tid < np) {
+      const int* el = sem + tid / NQ * ES;
+      const int t = shift(eg, el);
+      semt[tid] = t;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) eg[c] = el[eD + c] + t;
 #pragma unroll
       for (int a = 0; a < NN; ++a)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          sg[tid * GS + a * 3 + c] = fx_make(G[c][a], eg);
+          sg[tid * GS + a * 3 + c] = fx_make(G[c][a], eg[c]);
           if constexpr (!F64) sv[tid * SV + a * 6 + c] = ff_split_rn_bits(G[c][a]).h;
         }
     }
   } else {
-    for (int t = tid; t < np * NN; t += NT) {
-      const int a = t / np, r = t - a * np;
+    for (int k = tid; k < np * NN; k += NT) {
+      const int a = k / np, r = k - a * np;
+      const int* el = sem + r / NQ * ES;
+      const int t = shift(semp + r * 3, el);
+      if (a == 0) semt[r] = t;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double x = g.geomG[(int64_t)(c * NN + a) * stride + e0 * NQ + r];
-        sg[r * GS + a * 3 + c] = fx_make(x, emg[r]);
+        sg[r * GS + a * 3 + c] = fx_make(x, el[eD + c] + t);
         if constexpr (!F64) sv[r * SV + a * 6 + c] = ff_split_rn_bits(x).h;
       }
     }
@@ -153,7 +184,8 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
     if (tid < np) {
       const fx* gp = sg + tid * GS;
       const fx* up = suf + tid / NQ * NDOF;
-      FxSum s[6] = {};
+      const int* eu = sem + tid / NQ * ES + eU;
+      FxSum s[9] = {};
 #pragma unroll
       for (int a = 0; a < NN; ++a) {
         const fx gx = gp[a * 3], gy = gp[a * 3 + 1], gz = gp[a * 3 + 2];
@@ -162,14 +194,20 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
         fx_fma(s[1], gy, uy);
         fx_fma(s[2], gz, uz);
         fx_fma(s[3], gy, ux);
-        fx_fma(s[3], gx, uy);
         fx_fma(s[4], gz, ux);
-        fx_fma(s[4], gx, uz);
         fx_fma(s[5], gz, uy);
-        fx_fma(s[5], gy, uz);
+        fx_fma(s[6], gx, uy);
+        fx_fma(s[7], gx, uz);
+        fx_fma(s[8], gy, uz);
       }
 #pragma unroll
-      for (int f = 0; f < 6; ++f) de[f] = fx_value(fx_int(s[f]), eg + emu[tid / NQ]);
+      for (int f = 0; f < 6; ++f) {
+        const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+        int em = eg[j] + eu[i];
+        int64_t v = fx_int(s[f], -1);
+        if (f >= 3) v = fx_add(v, em, fx_int(s[f + 3], -1), eg[i] + eu[j]);
+        de[f] = fx_value(v, em + 1);
+      }
     }
   } else {
     for (int t = tid; t < np * 6; t += NT) {
@@ -182,7 +220,10 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
         fx_fma(s, gp[a * 3 + j], up[a * 3 + i]);
         if (f >= 3) fx_fma(s2, gp[a * 3 + i], up[a * 3 + j]);
       }
-      sd[r * DS + f] = fx_value(fx_int(s, -1) + fx_int(s2, -1), emg[r] + emu[r / NQ] + 1);
+      const int *el = sem + r / NQ * ES, t0 = semt[r];
+      int em = el[eD + j] + el[eU + i] + t0;
+      const int64_t v = fx_add(fx_int(s, -1), em, fx_int(s2, -1), f >= 3 ? el[eD + i] + el[eU + j] + t0 : em);
+      sd[r * DS + f] = fx_value(v, em + 1);
     }
     __syncthreads();
   }
@@ -210,28 +251,38 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
     else
       ok = von_mises_3d_f32(smc[le], sig, de, kappa, T);
     bool finite = true;
-    int es = 0;
+    int* el = sem + le * ES;
+    const int t0 = semt[t];
+    int es[3] = {0, 0, 0};
     for (int f = 0; f < 6; ++f) {
       g.stateTemp[(int64_t)f * stride + pt] = sig[f];
       g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
       finite = finite && finite_bits(sig[f]);
       const double ss = sig[f] * s;
       sd[t * DS + f] = ss;
-      es = fx_max_exponent(es, ss);
+      const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2), ef = fx_exponent(ss);
+      es[i] = max(es[i], ef + el[eD + j]);
+      es[j] = max(es[j], ef + el[eD + i]);
     }
     if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
     if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
     if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
-    atomicMax(ems + le, es + emg[t]);
+    for (int c = 0; c < 3; ++c) atomicMax(el + eE + c, es[c] + t0);
     const double c[3] = {T.c12 * s, T.c44 * s, T.a * s};
     if constexpr (F64) {
-      for (int f = 0; f < 6; ++f) sn[t * DS + f] = T.n[f];
-      for (int k = 0; k < 3; ++k) sc[t * 3 + k] = c[k];
-      int ea = fx_exponent(c[2]);
-      for (int f = 0; f < 6; ++f)
-        if (fx_exponent(T.n[f]) >= FX_NAN) ea = FX_NAN;
-      atomicMax(emc + le, max(fx_exponent(c[0]), fx_exponent(c[1])) + 2 * emg[t]);
-      atomicMax(ema + le, ea + 2 * emg[t]);
+      int ez[3] = {0, 0, 0};
+      for (int f = 0; f < 6; ++f) {
+        sn[t * DS + f] = T.n[f];
+        const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2), ef = fx_exponent(T.n[f]);
+        ez[i] = max(ez[i], ef + el[eD + j]);
+        ez[j] = max(ez[j], ef + el[eD + i]);
+      }
+      for (int k = 0; k < 3; ++k) {
+        sc[t * 3 + k] = c[k];
+        atomicMax(el + eZ + k, ez[k]);
+      }
+      atomicMax(el + eC, max(fx_exponent(c[0]), fx_exponent(c[1])) + 2 * t0);
+      atomicMax(el + eA, fx_exponent(c[2]) + 2 * t0);
     } else {
       for (int k = 0; k < 3; ++k) sc[t * 3 + k] = ff_split_rn_bits(c[k]).h;
       const float* n = T.n;
@@ -252,14 +303,15 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
 
   // ---- digits of the per-point factors
   for (int t = tid; t < np * 6; t += NT) {
-    const int r = t / 6, i = r * DS + (t - r * 6);
-    sdf[i] = fx_make(sd[i], ems[r / NQ] - emg[r]);
-    if constexpr (F64) snf[i] = fx_make(sn[i], 1023);
+    const int r = t / 6, f = t - r * 6;
+    const int* el = sem + r / NQ * ES;
+    row_digits(sdf + r * DS, sd[r * DS + f], f, el + eE, el + eD, semt[r]);
+    if constexpr (F64) row_digits(snf + r * DS, sn[r * DS + f], f, el + eZ, el + eD, 0);
   }
   if constexpr (F64) {
     for (int t = tid; t < np * 3; t += NT) {
       const int r = t / 3;
-      scf[t] = fx_make(sc[t], (t - r * 3 == 2 ? ema : emc)[r / NQ] - 2 * emg[r]);
+      scf[t] = fx_make(sc[t], sem[r / NQ * ES + (t - r * 3 == 2 ? eA : eC)] - 2 * semt[r]);
     }
   }
   if constexpr (F64 || !PERPOINT) {
@@ -271,21 +323,18 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
         const fx gx = sg[r * GS + a * 3], gy = sg[r * GS + a * 3 + 1], gz = sg[r * GS + a * 3 + 2];
         const fx* n = snf + r * DS;
         FxSum z[3] = {};
-        fx_fma(z[0], n[0], gx);
-        fx_fma(z[0], n[3], gy);
-        fx_fma(z[0], n[4], gz);
-        fx_fma(z[1], n[3], gx);
-        fx_fma(z[1], n[1], gy);
-        fx_fma(z[1], n[5], gz);
-        fx_fma(z[2], n[4], gx);
-        fx_fma(z[2], n[5], gy);
-        fx_fma(z[2], n[2], gz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          fx_fma(z[c], n[row_slot(c, 0)], gx);
+          fx_fma(z[c], n[row_slot(c, 1)], gy);
+          fx_fma(z[c], n[row_slot(c, 2)], gz);
+        }
         const fx c0 = scf[r * 3], c1 = scf[r * 3 + 1], c2 = scf[r * 3 + 2];
         fx* v = sset + (size_t)r * GS + a * 3;
         const fx gv[3] = {gx, gy, gz};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const fx zc = fx_split(fx_int(z[c], -1));  // scale em_g + 1: |n| <= 1, the row of n at most 1 long
+          const fx zc = fx_split(fx_int(z[c], -3));  // three products: scale Z_c + t - 1020
           v[c] = fx_mul(c0, gv[c]);
           v[(size_t)NP * GS + c] = fx_mul(c1, gv[c]);
           v[(size_t)2 * NP * GS + c] = fx_mul(c2, zc);
@@ -307,7 +356,7 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
   for (int t = tid; t < nLoc * NDOF; t += NT) {
     const int le = t / NDOF, k = t - le * NDOF, a = k / 3, c = k - 3 * a;
     const int64_t e = e0 + le;
-    const int v0 = c == 0 ? 0 : c + 2, v1 = c == 0 ? 3 : (c == 1 ? 1 : 5), v2 = c == 0 ? 4 : (c == 1 ? 5 : 2);
+    const int v0 = row_slot(c, 0), v1 = row_slot(c, 1), v2 = row_slot(c, 2);
     constexpr int R = NQ > 8 ? -2 : 0;
     FxSum s[3] = {};  // one for each direction: 27 products at most
     for (int q = 0; q < NQ; ++q) {
@@ -317,7 +366,7 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
       fx_fma(s[1], dp[v1], gp[1]);
       fx_fma(s[2], dp[v2], gp[2]);
     }
-    const double pe = -fx_value(fx_int(s[0], R) + fx_int(s[1], R) + fx_int(s[2], R), ems[le] - R);
+    const double pe = -fx_value(fx_int(s[0], R) + fx_int(s[1], R) + fx_int(s[2], R), sem[le * ES + eE + c] - R);
     const int32_t node = g.conn[e * NN + a];
     if (!in_bounds(g, node, g.nNodes, e)) continue;
     const int32_t dof = g.nodeDof[node] + c;
@@ -357,24 +406,29 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
           }
         }
       }
-      // The first two sums in units of em_c - 1022, the third of em_a - 1022 + 2, added at the coarser of the two with
-      // B guard bits: as many as the largest of the 27 sums leaves (six of them add up)
+      // The first two sums in units of em_c - 1022 + D_j + D_k, the third of em_a - 3062 + Z_j + Z_k, added at the coarser
+      // of them with B guard bits: as many as the largest of the 27 sums leaves (six of them add up)
       int top = 0;
 #pragma unroll
       for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int k = 0; k < 3; ++k) top |= fx_bits(s1[j][k]) | fx_bits(s2[j][k]) | fx_bits(s3[j][k]);
       const int B = min(__clz(top) - 5, 26);
-      const int64_t dot = fx_int(s2[0][0], B) + fx_int(s2[1][1], B) + fx_int(s2[2][2], B);
-      const int ec = emc[le] - 1022, ea = ema[le] - 1020, d = ea - ec;
-      const int em = emc[le] >= FX_NAN || ema[le] >= FX_NAN ? FX_NAN : max(ec, ea) - B;
-      const int dc = min(max(d, 0), 63), da = min(max(-d, 0), 63);
+      const int* el = sem + le * ES;
+      const int ec = el[eC] - 1022, ea = el[eA] - 3062, D[3] = {el[eD], el[eD + 1], el[eD + 2]}, Z[3] = {el[eZ], el[eZ + 1], el[eZ + 2]};
+      const int Dm = max(D[0], max(D[1], D[2]));
+      int64_t dot = 0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dot += fx_down(fx_int(s2[j][j], B), 2 * (Dm - D[j]));
 #pragma unroll
       for (int j = 0; j < 3; ++j)
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-          acc[j][k] = fx_value(fx_shift(fx_int(s1[j][k], B) + fx_int(s2[k][j], B) + (j == k ? dot : 0), dc) -
-                                   fx_shift(fx_int(s3[j][k], B), da), em);
+        for (int k = 0; k < 3; ++k) {
+          const int cjk = ec + D[j] + D[k], ajk = ea + Z[j] + Z[k], em = max(j == k ? ec + 2 * Dm : cjk, ajk);
+          int64_t v = fx_down(fx_int(s1[j][k], B) + fx_int(s2[k][j], B), em - cjk) - fx_down(fx_int(s3[j][k], B), em - ajk);
+          if (j == k) v += fx_down(dot, em - ec - 2 * Dm);
+          acc[j][k] = fx_value(v, em - B);
+        }
     } else {
 #pragma unroll
       for (int j = 0; j < 3; ++j)
@@ -418,7 +472,7 @@ __device__ __forceinline__ void assemble_tile_ss3(const GroupArgs& g, const int6
 // element also holding its eight nodes.  The scales are maxima and the residual a transposing sum over eight lanes;
 // the point's row of shared memory holds the digits of dN/dX and then, in their place, the tangent's vectors.  The only
 // wait for other warps is for the elements' material constants (FP64 divisions, formed by one warp for all).  262144
-// elements: 995 us; latency of the chain through a warp's phases binds it (the FP64
+// elements: 992 us; latency of the chain through a warp's phases binds it (the FP64
 // pipe is about half busy), hence few registers and 24 warps per SM.
 template <int NT>
 struct SS3Hexa8Layout {
@@ -450,9 +504,10 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
 
   // ---- the node's dU relative to the element's first node, digits of it and of the point's dN/dX
   int32_t dof = -1;
-  int eg = 0, eu = 0;
+  int eg[3] = {0, 0, 0}, eu[3] = {0, 0, 0};  // scales of the point's dN/dX and of dU
   {
     double u[3] = {0.0, 0.0, 0.0};
+    double G[3][NN];
     int rl = 0;
     if (live) {
       const int32_t node = g.conn[e * NN + q];
@@ -465,7 +520,6 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
           for (int c = 0; c < 3; ++c) u[c] = g.dU[d + c];
         }
       }
-      double G[3][NN];
       const double* gp = g.geomG + pt;
 #pragma unroll
       for (int c = 0; c < 3; ++c)
@@ -474,27 +528,36 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int a = 0; a < NN; ++a) eg = fx_max_exponent(eg, G[c][a]);
-#pragma unroll
-      for (int a = 0; a < NN; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) row[a * 3 + c] = fx_make(G[c][a], eg);
+        for (int a = 0; a < NN; ++a) eg[c] = fx_max_exponent(eg[c], G[c][a]);
     }
     srl[lane] = rl;
+    int D[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       u[c] -= __shfl_sync(0xffffffffu, u[c], lane & 24);
-      eu = fx_max_exponent(eu, u[c]);
+      eu[c] = fx_exponent(u[c]);
+      D[c] = eg[c];
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        eu[c] = max(eu[c], __shfl_xor_sync(0xffffffffu, eu[c], o));
+        D[c] = max(D[c], __shfl_xor_sync(0xffffffffu, D[c], o));
+      }
+      su[lane * 3 + c] = fx_make(u[c], eu[c]);
     }
+    if (live) {
+      const int t = max(max(eg[0] - D[0], eg[1] - D[1]), eg[2] - D[2]);
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) eu = max(eu, __shfl_xor_sync(0xffffffffu, eu, o));
+      for (int c = 0; c < 3; ++c) eg[c] = D[c] + t;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) su[lane * 3 + c] = fx_make(u[c], eu);
+      for (int a = 0; a < NN; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) row[a * 3 + c] = fx_make(G[c][a], eg[c]);
+    }
   }
   __syncthreads();
 
   // ---- strain increment (element.py:322), material update, state
-  int es = 0, ep = 0;  // scales of s sigma (times dN/dX), of sigma
+  int es[3] = {0, 0, 0};  // scales of the residual's rows
   double sig[6] = {0, 0, 0, 0, 0, 0}, s = 0.0;
   float n[6], cf[3];
   if (live) {
@@ -505,7 +568,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
     const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
     if (hasM) kappa = g.stateRef[(int64_t)12 * stride + pt];
     {
-      FxSum acc[6] = {};
+      FxSum acc[9] = {};
       const fx* up = su + le * 24;
 #pragma unroll
       for (int a = 0; a < NN; ++a) {
@@ -515,14 +578,20 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
         fx_fma(acc[1], gy, uy);
         fx_fma(acc[2], gz, uz);
         fx_fma(acc[3], gy, ux);
-        fx_fma(acc[3], gx, uy);
         fx_fma(acc[4], gz, ux);
-        fx_fma(acc[4], gx, uz);
         fx_fma(acc[5], gz, uy);
-        fx_fma(acc[5], gy, uz);
+        fx_fma(acc[6], gx, uy);
+        fx_fma(acc[7], gx, uz);
+        fx_fma(acc[8], gy, uz);
       }
 #pragma unroll
-      for (int f = 0; f < 6; ++f) de[f] = fx_value(fx_int(acc[f]), eg + eu);
+      for (int f = 0; f < 6; ++f) {
+        const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+        int em = eg[j] + eu[i];
+        int64_t v = fx_int(acc[f], -1);
+        if (f >= 3) v = fx_add(v, em, fx_int(acc[f + 3], -1), eg[i] + eu[j]);
+        de[f] = fx_value(v, em + 1);
+      }
     }
     bool ok = true;
     TangentF32 T;
@@ -540,31 +609,48 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
       g.stateTemp[(int64_t)f * stride + pt] = sig[f];
       g.stateTemp[(int64_t)(6 + f) * stride + pt] = de[f];
       finite = finite && finite_bits(sig[f]);
-      ep = fx_max_exponent(ep, sig[f]);
       n[f] = T.n[f];
     }
     if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
     if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
     if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
-    es = ep + fx_exponent(s) - 1022 + eg;
     cf[0] = ff_split_rn_bits(T.c12 * s).h;
     cf[1] = ff_split_rn_bits(T.c44 * s).h;
     cf[2] = ff_split_rn_bits(T.a * s).h;
   }
   // ---- residual: s sigma . G_a of the point for every node, summed over the element's points by exchanges that leave
   // node q's three sums in lane q
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) es = max(es, __shfl_xor_sync(0xffffffffu, es, o));
   {
-    const fx sd = fx_make(s, es - eg - ep + 1022);  // s sigma at the scale es - eg
-    fx d[6];
+    // s sigma exactly as integers, then their digits in the rows' scales
+    const int e1 = fx_exponent(s) - 1022;  // of s sigma: that of sigma and this
+    int ef[6];
+    fx d[9];
 #pragma unroll
-    for (int f = 0; f < 6; ++f) d[f] = fx_mul(fx_make(sig[f], ep), sd);  // zero in lanes without a point
+    for (int f = 0; f < 6; ++f) {
+      const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+      ef[f] = fx_exponent(sig[f]) + e1;
+      es[i] = max(es[i], ef[f] + eg[j]);
+      es[j] = max(es[j], ef[f] + eg[i]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) es[c] = max(es[c], __shfl_xor_sync(0xffffffffu, es[c], o));
+    const fx sd = fx_make(s, e1 + 1022);
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
+      FxSum p{0, 0};
+      fx_fma(p, fx_make(sig[f], ef[f] - e1), sd);
+      const int64_t v = live ? fx_int(p, -1) : 0;
+      d[f] = fx_split(fx_shift(v, min(es[i] - eg[j] - ef[f], 62)));  // rounded: an operand
+      if (f >= 3) d[f + 3] = fx_split(fx_shift(v, min(es[j] - eg[i] - ef[f], 62)));
+    }
     auto force = [&](int a, int c) {
       FxSum r{0, 0};
-      fx_fma(r, d[c == 0 ? 0 : c + 2], row[a * 3]);
-      fx_fma(r, d[c == 0 ? 3 : (c == 1 ? 1 : 5)], row[a * 3 + 1]);
-      fx_fma(r, d[c == 0 ? 4 : (c == 1 ? 5 : 2)], row[a * 3 + 2]);
+      fx_fma(r, d[row_slot(c, 0)], row[a * 3]);
+      fx_fma(r, d[row_slot(c, 1)], row[a * 3 + 1]);
+      fx_fma(r, d[row_slot(c, 2)], row[a * 3 + 2]);
       return (long long)fx_int(r);
     };
     if (!live)
@@ -582,7 +668,7 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
       }
       const long long x0 = (b1 ? t[2] : t[0]) + __shfl_xor_sync(0xffffffffu, b1 ? t[0] : t[2], 2);
       const long long x1 = (b1 ? t[3] : t[1]) + __shfl_xor_sync(0xffffffffu, b1 ? t[1] : t[3], 2);
-      pe[c] = -fx_value((b0 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b0 ? x0 : x1, 1), es);
+      pe[c] = -fx_value((b0 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b0 ? x0 : x1, 1), es[c]);
     }
     if (dof >= 0) {
 #pragma unroll
@@ -592,12 +678,13 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
       }
     }
   }
-  // ---- the tangent's vectors in the place of the digits: the upper digit has 29 bits, more than a float
+  // ---- the tangent's vectors in the place of the digits, from the upper ones: 29 bits of the largest of their component.
+  // The FP32 sums round at 24 of it: errors of K with all bits, or with dN/dX itself rounded, are the same within 1 %.
   if (live) {
-    const float sc = eg >= FX_NAN ? __int_as_float(0x7fc00000) : (float)scalbn(1.0, max(-300, min(300, eg - 1051)));
+    const float sx = fx_unit(eg[0]), sy = fx_unit(eg[1]), sz = fx_unit(eg[2]);
 #pragma unroll
     for (int a = 0; a < NN; ++a) {
-      const float gx = (float)row[a * 3].h * sc, gy = (float)row[a * 3 + 1].h * sc, gz = (float)row[a * 3 + 2].h * sc;
+      const float gx = fx_float(row[a * 3], sx), gy = fx_float(row[a * 3 + 1], sy), gz = fx_float(row[a * 3 + 2], sz);
       float2* v = reinterpret_cast<float2*>(row + a * 3);
       v[0] = make_float2(gx, gy);
       v[1] = make_float2(gz, n[0] * gx + n[3] * gy + n[4] * gz);
@@ -665,28 +752,33 @@ __device__ __forceinline__ void assemble_tile_ss3_hexa8(const GroupArgs& g, cons
 // g = F dN/dX: with c1 = sB and c3 = c4 in every variant, B h = g and dN_a/dX . dN_b/dX = h_a . g_b,
 //   K_ab[j][k] = sum_q s (c2 h_a[j] h_b[k] + c3 (g_a[j] h_b[k] + h_a[j] g_b[k]) - sI h_a[k] h_b[j] + c1 delta_jk h_a . g_b).
 //
-// 13824 elements: small strain (von Mises) 678 -> 380 us, where a tensor-core tile (tcgen05, TF32 hi/lo) ran; TL 704 ->
-// 467 us, mixed-ff 665 -> 468 us, against the same.  That tile's serial phases (operand conversion, FP64 update on one
+// 13824 elements: small strain (von Mises) 675 -> 383 us, where a tensor-core tile (tcgen05, TF32 hi/lo) ran; TL 704 ->
+// 463 us, mixed-ff 606 -> 463 us, against the same.  That tile's serial phases (operand conversion, FP64 update on one
 // warp, MMA waits) with twelve warps per SM bound it, not the products; its tangent was 8e-7 off, this one 7e-8.  Here
 // the issue slots (63 % used, small strain) and the waits of the phases with a thread per point bind.
 template <bool TL>
 struct Hexa20Layout {
   static constexpr int EPB = 2, NT = 128, NN = 20, NQ = 27, NDOF = 60, NP = EPB * NQ, NB = 55;  // NB: node blocks A <= B
   // a point's row in doublewords: 60 digits, then the floats (dN/dX, n dN/dX) of 20 nodes; odd
-  static constexpr int SV = 61, DS = TL ? 9 : 7, SN = TL ? 19 : 7, SK = 61;
+  static constexpr int SV = 61, DS = 9, SN = TL ? 21 : 9, SK = 61;
   static constexpr size_t v_off = 0;                            // fx [NP][SV]
   static constexpr size_t u_off = v_off + 8 * NP * SV;          // fx [EPB][NDOF]
   static constexpr size_t d_off = u_off + 8 * EPB * NDOF;       // int64 [NP][DS]: half of the strain (H); fx: s sigma (s P)
   static constexpr size_t k_bytes = 4 * EPB * NDOF * SK;        // K_e, in their place: float [EPB][NDOF][SK]
   static_assert(k_bytes <= d_off + 8 * NP * DS, "K_e fits the area of the operands");
-  static constexpr size_t c_off = (d_off + 8 * NP * DS + 15) / 16 * 16;  // float4 [NP]: coefficients (small strain: and the unit)
-  // float [NP][SN]: flow direction, or F^-1, F and the unit of the upper digits
+  static constexpr size_t c_off = (d_off + 8 * NP * DS + 15) / 16 * 16;  // float4 [NP]: coefficients of the tangent
+  // float [NP][SN]: flow direction, or F^-1 and F, and the units of dN/dX's digits
   static constexpr size_t n_off = c_off + 16 * NP;
   static constexpr size_t mc_off = (n_off + 4 * NP * SN + 15) / 16 * 16;  // VMConst [EPB]
   static constexpr size_t sl_off = mc_off + sizeof(VMConst) * EPB;        // int [EPB][NN][NN]: pair slots
   static constexpr size_t rl_off = sl_off + 4 * EPB * NN * NN;            // int [EPB][NN]: row lengths
-  static constexpr size_t e_off = rl_off + 4 * EPB * NN;                  // int [2][NP]: halves of em_g; [EPB]: em_u, em_s
-  static constexpr size_t bytes = e_off + 4 * (2 * NP + 2 * EPB);
+  // int [4 warps][EPB][3]: an element's maxima; [EPB][3]: scales of dU, of the residual's rows
+  static constexpr size_t e_off = rl_off + 4 * EPB * NN;
+  static constexpr size_t bytes = e_off + 4 * 18 * EPB;
+  // before the flow direction, in its place: int [NP][4]: a point's maxima (of 1, two halves of 2, of 3); [NP][3]: scales of
+  // its dN/dX
+  static_assert(SN >= 7, "scales in the place of the flow direction");
+  static_assert(TL || 5 * (bytes + 1024) <= 196 * 1024, "the rest of the SM's 256 KB is L1 in steps: above this 28 KB instead of 60");
 };
 
 // Total-Lagrangian Neo-Hooke update of one point from H (displacementtlelement/element.py:386-414): state, strain, s P =
@@ -764,8 +856,8 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
   VMConst* smc = reinterpret_cast<VMConst*>(smem + L::mc_off);
   int* sps = reinterpret_cast<int*>(smem + L::sl_off);
   int* srl = reinterpret_cast<int*>(smem + L::rl_off);
-  int* sem = reinterpret_cast<int*>(smem + L::e_off);
-  int *emu = sem + 2 * NP, *ems = emu + EPB;
+  int *sem = reinterpret_cast<int*>(sn), *semG = sem + 4 * NP;
+  int *semD = reinterpret_cast<int*>(smem + L::e_off), *emu = semD + 12 * EPB, *ems = emu + 3 * EPB;
   const int64_t nEl = g.nElements, stride = nEl * NQ;
   const int nLoc = nEl - e0 < EPB ? (int)(nEl - e0) : EPB;
   const bool vm = g.material == EFE_MAT_VON_MISES;
@@ -778,7 +870,6 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
     const bool live = part < 2 && r < nLoc * NQ;
     constexpr int H = NDOF / 2;
     double G[H];
-    int em = 0;
     if (live) {
       const double* gp = g.geomG + (int64_t)(part * H) * stride + e0 * NQ + r;
 #pragma unroll
@@ -787,7 +878,6 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
     const int le = wid;
     if (le < EPB) {
       double u[3] = {0.0, 0.0, 0.0};
-      int eu = 0;
       const int64_t e = e0 + le;
       if (lane < NN && le < nLoc) {
         const int32_t node = g.conn[e * NN + lane], node0 = g.conn[e * NN];
@@ -797,36 +887,55 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
           const int32_t dof = g.nodeDof[node], dof0 = g.nodeDof[node0];
           if (in_bounds(g, dof, g.nDof - 2, e) && in_bounds(g, dof0, g.nDof - 2, e)) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              u[c] = Ux[dof + c] - Ux[dof0 + c];
-              eu = fx_max_exponent(eu, u[c]);
-            }
+            for (int c = 0; c < 3; ++c) u[c] = Ux[dof + c] - Ux[dof0 + c];
           }
         }
         srl[le * NN + lane] = rl;
       }
-      eu = __reduce_max_sync(0xffffffffu, eu);
-      if (lane < NN)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) su[le * NDOF + lane * 3 + c] = fx_make(u[c], eu);
-      if (lane == 0) emu[le] = eu;
+      for (int c = 0; c < 3; ++c) {
+        const int eu = __reduce_max_sync(0xffffffffu, fx_exponent(u[c]));
+        if (lane < NN) su[le * NDOF + lane * 3 + c] = fx_make(u[c], eu);
+        if (lane == 0) emu[le * 3 + c] = eu;
+      }
     }
+    // the first part's values are component 0 of all nodes and 1 of ten, the second's 1 of the others and 2 of all
+    int em0 = 0, em1 = 0;
     if (live) {
+      int m[3] = {0, 0, 0};
 #pragma unroll
-      for (int i = 0; i < H; ++i) em = fx_max_exponent(em, G[i]);
-      sem[part * NP + r] = em;
+      for (int i = 0; i < H; ++i) m[i / 10] = fx_max_exponent(m[i / 10], G[i]);
+      em0 = part ? m[0] : max(m[0], m[1]);
+      em1 = part ? max(m[1], m[2]) : m[2];
+      sem[r * 4 + part * 2] = em0;
+      sem[r * 4 + part * 2 + 1] = em1;
     }
+#pragma unroll
+    for (int el = 0; el < EPB; ++el)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const bool mine = live && r / NQ == el && (c == 1 || c == 2 * part);
+        const int m = __reduce_max_sync(0xffffffffu, mine ? (c == part ? em0 : em1) : 0);
+        if (lane == 0) semD[(wid * EPB + el) * 3 + c] = m;
+      }
     if (!TL && wid == 3 && lane >= 32 - nLoc) {
       const int k = 31 - lane;
       smc[k] = vm_const<true>(g.props + (e0 + k) * g.nProps, vm);
     }
     __syncthreads();
     if (live) {
-      em = max(sem[r], sem[NP + r]);
+      const int *pm = sem + r * 4, *dm = semD + r / NQ * 3;
+      int D[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) D[c] = max(max(dm[c], dm[3 * EPB + c]), max(dm[6 * EPB + c], dm[9 * EPB + c]));
+      const int t = max(max(pm[0] - D[0], max(pm[1], pm[2]) - D[1]), pm[3] - D[2]);
+      if (part == 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) semG[r * 3 + c] = D[c] + t;
 #pragma unroll
       for (int i = 0; i < H; ++i) {
         const int la = part * H + i, c = la / NN, a = la - c * NN;
-        sv[r * SV + a * 3 + c] = fx_make(G[i], em);
+        sv[r * SV + a * 3 + c] = fx_make(G[i], (i < 10 ? (part ? D[1] : D[0]) : i < 20 ? (part ? D[2] : D[0]) : (part ? D[2] : D[1])) + t);
       }
     }
   }
@@ -835,7 +944,13 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
   // ---- strain increment (element.py:322): two warps per element, a lane per point, ten nodes each
   const int le = wid >> 1, half = wid & 1, pr = le * NQ + lane;
   const bool live = le < nLoc && lane < NQ;
-  const int eg = live ? max(sem[pr], sem[NP + pr]) : 0;
+  int eg[3] = {0, 0, 0}, eu[3] = {0, 0, 0};
+  if (live)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      eg[c] = semG[pr * 3 + c];
+      eu[c] = emu[le * 3 + c];
+    }
   const int64_t e = e0 + le, pt = e * NQ + lane;
   const bool hasM = g.material != EFE_MAT_LINEAR_ELASTIC;
   constexpr int NS = TL ? 9 : 6;
@@ -850,7 +965,7 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
     s = g.geomS[pt];
   }
   if (live) {
-    FxSum acc[NS] = {};
+    FxSum acc[9] = {};
     const fx *gp = sv + pr * SV + half * 30, *up = su + le * NDOF + half * 30;
 #pragma unroll 5
     for (int a = 0; a < NN / 2; ++a) {
@@ -865,16 +980,21 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
         fx_fma(acc[1], G[1], u[1]);
         fx_fma(acc[2], G[2], u[2]);
         fx_fma(acc[3], G[1], u[0]);
-        fx_fma(acc[3], G[0], u[1]);
         fx_fma(acc[4], G[2], u[0]);
-        fx_fma(acc[4], G[0], u[2]);
         fx_fma(acc[5], G[2], u[1]);
-        fx_fma(acc[5], G[1], u[2]);
+        fx_fma(acc[6], G[0], u[1]);
+        fx_fma(acc[7], G[0], u[2]);
+        fx_fma(acc[8], G[1], u[2]);
       }
     }
 #pragma unroll
     for (int f = 0; f < NS; ++f) {
+      const int i = f < 3 ? f : (f == 5 ? 1 : 0), j = f < 3 ? f : (f == 3 ? 1 : 2);
       st[f] = fx_int(acc[f], -1);
+      if (!TL && f >= 3) {
+        int em = eg[j] + eu[i];
+        st[f] = fx_add(st[f], em, fx_int(acc[f + 3], -1), eg[i] + eu[j]);
+      }
       if (half) sde[pr * DS + f] = st[f];
     }
   }
@@ -882,16 +1002,17 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
 
   // ---- material points: one warp of each element
   if (half == 0) {
-    int es = 0;
+    int es[3] = {0, 0, 0};
     double ss[NS] = {};  // s sigma, or s P = s tau F^-T
-    // the upper digits of dN/dX have 29 bits, more than a float
-    auto unit = [&] { return eg >= FX_NAN ? __int_as_float(0x7fc00000) : ldexpf(1.0f, max(-300, min(300, eg - 1051))); };
     if (live) {
       double de[NS];  // the strain increment, or H
 #pragma unroll
-      for (int f = 0; f < NS; ++f) de[f] = fx_value(st[f] + sde[pr * DS + f], eg + emu[le] + 1);
+      for (int f = 0; f < NS; ++f) {
+        const int i = TL ? f / 3 : f < 3 ? f : (f == 5 ? 1 : 0), j = TL ? f % 3 : f < 3 ? f : (f == 3 ? 1 : 2);
+        const int em = TL || f < 3 ? eg[j] + eu[i] : max(eg[j] + eu[i], eg[i] + eu[j]);
+        de[f] = fx_value(st[f] + sde[pr * DS + f], em + 1);
+      }
       if constexpr (TL) {
-        sn[pr * SN + 18] = unit();
         hexa20_neo_hooke(g, e, pt, stride, s, de, ss, sc + pr, sn + pr * SN);
       } else {
         double eps[6];
@@ -910,27 +1031,50 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
           g.stateTemp[(int64_t)(6 + f) * stride + pt] = eps[f] + de[f];
           finite = finite && finite_bits(sig[f]);
           ss[f] = s * sig[f];
-          es = fx_max_exponent(es, ss[f]);
           sn[pr * SN + f] = T.n[f];
         }
         if (hasM) g.stateTemp[(int64_t)12 * stride + pt] = kappa;
         if (!ok) report(g.status, EFE_STATUS_CUTBACK, g.elementOffset + e, 1);
         if (!finite) atomicOr(g.status, EFE_STATUS_NONFINITE);
         sc[pr] = make_float4(ff_split_rn_bits(T.c12 * s).h, ff_split_rn_bits(T.c44 * s).h, ff_split_rn_bits(T.a * s).h,
-                             unit());
+                             0.0f);
       }
-      if constexpr (TL)
 #pragma unroll
-        for (int f = 0; f < NS; ++f) es = fx_max_exponent(es, ss[f]);
-      es += eg;
+      for (int f = 0; f < NS; ++f) {
+        const int i = TL ? f / 3 : f < 3 ? f : (f == 5 ? 1 : 0), j = TL ? f % 3 : f < 3 ? f : (f == 3 ? 1 : 2);
+        const int ef = fx_exponent(ss[f]);
+        es[i] = max(es[i], ef + eg[j]);
+        if (!TL) es[j] = max(es[j], ef + eg[i]);
+      }
     }
-    es = __reduce_max_sync(0xffffffffu, es);
-    if (lane == 0) ems[le] = es;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      es[c] = __reduce_max_sync(0xffffffffu, es[c]);
+      if (lane == 0) ems[le * 3 + c] = es[c];
+    }
     if (live)
 #pragma unroll
-      for (int f = 0; f < NS; ++f) sd[pr * DS + f] = fx_make(ss[f], es - eg);
+      for (int f = 0; f < NS; ++f) {
+        if constexpr (TL)
+          sd[pr * DS + f] = fx_make(ss[f], es[f / 3] - eg[f % 3]);
+        else
+          reinterpret_cast<double*>(sd)[pr * DS + f] = ss[f];
+      }
+  } else if (live) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sn[pr * SN + SN - 3 + c] = fx_unit(eg[c]);
   }
   __syncthreads();
+  // small strain: digits of the nine row factors by both warps (13824 elements: 12 us less than by one)
+  if constexpr (!TL) {
+    if (live) {
+      const int es[3] = {ems[le * 3], ems[le * 3 + 1], ems[le * 3 + 2]};
+#pragma unroll
+      for (int f = 0; f < NS; ++f)
+        if ((f >= 4) == half) row_digits(sd + pr * DS, reinterpret_cast<const double*>(sd)[pr * DS + f], f, es, eg, 0);
+    }
+    __syncthreads();
+  }
 
   // ---- residual and flux (NIST.computeElements, nonlinearimplicitstatic.py:837-844): 60 threads per element
   {
@@ -938,8 +1082,7 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
     if (k < NDOF && el < nLoc) {
       const int a = k / 3, c = k - 3 * a;
       const int64_t e = e0 + el;
-      const int v0 = TL ? 3 * c : (c == 0 ? 0 : c + 2), v1 = TL ? 3 * c + 1 : (c == 0 ? 3 : (c == 1 ? 1 : 5)),
-                v2 = TL ? 3 * c + 2 : (c == 0 ? 4 : (c == 1 ? 5 : 2));
+      const int v0 = TL ? 3 * c : row_slot(c, 0), v1 = TL ? 3 * c + 1 : row_slot(c, 1), v2 = TL ? 3 * c + 2 : row_slot(c, 2);
       FxSum s[3] = {};  // one for each direction: 27 products
       const fx *gp = sv + el * NQ * SV + a * 3, *dp = sd + el * NQ * DS;
 #pragma unroll 3
@@ -948,7 +1091,7 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
         fx_fma(s[1], dp[q * DS + v1], gp[q * SV + 1]);
         fx_fma(s[2], dp[q * DS + v2], gp[q * SV + 2]);
       }
-      const double pe = -fx_value(fx_int(s[0], -2) + fx_int(s[1], -2) + fx_int(s[2], -2), ems[el] + 2);
+      const double pe = -fx_value(fx_int(s[0], -2) + fx_int(s[1], -2) + fx_int(s[2], -2), ems[el * 3 + c] + 2);
       const int32_t node = g.conn[e * NN + a];
       if (in_bounds(g, node, g.nNodes, e)) {
         const int32_t dof = g.nodeDof[node] + c;
@@ -961,16 +1104,16 @@ __device__ __forceinline__ void assemble_tile_hexa20(const GroupArgs& g, const i
   }
   __syncthreads();
 
-  // ---- the tangent's vectors in the place of the digits
+  // ---- the tangent's vectors in the place of the digits (as in the Hexa8 tile)
   if (live) {
-    const float unit = TL ? sn[pr * SN + 18] : sc[pr].w;
+    const float *unit = sn + pr * SN + SN - 3, ux = unit[0], uy = unit[1], uz = unit[2];
     float n[TL ? 18 : 6];
 #pragma unroll
     for (int f = 0; f < (TL ? 18 : 6); ++f) n[f] = sn[pr * SN + f];
     fx* row = sv + pr * SV + half * 30;
 #pragma unroll 5
     for (int a = 0; a < NN / 2; ++a) {
-      const float gx = (float)row[a * 3].h * unit, gy = (float)row[a * 3 + 1].h * unit, gz = (float)row[a * 3 + 2].h * unit;
+      const float gx = fx_float(row[a * 3], ux), gy = fx_float(row[a * 3 + 1], uy), gz = fx_float(row[a * 3 + 2], uz);
       float x[6];
       if constexpr (TL) {
 #pragma unroll
