@@ -21,6 +21,8 @@ import torch
 
 from .exceptions import CutbackRequest
 
+LAUNCH_SECONDS = 20e-3  # of CG iterations in one launch: what the host's look at the outcome costs is small beside it
+
 TimeStep = namedtuple("TimeStep", "number stepProgressIncrement stepProgress timeIncrement stepTime totalTime")
 
 
@@ -398,9 +400,9 @@ class NISTGPU:
         k = 0
         if bnorm > 0.0 and float(work[2]) > tol2:
             cols = ctypes.c_void_p(self._block_cols.data_ptr() if self._block_cols is not None else None)
-            # one launch runs about 20 ms of iterations (and returns early once the solve has ended)
+            # one launch runs 50 iterations or LAUNCH_SECONDS of them (and returns early once the solve has ended)
             seconds = 4e-6 + asm.nnz * K.element_size() / 4e12
-            segment = 10 * min(200, max(5, int(2e-3 / seconds)))
+            segment = 10 * min(200, max(5, int(0.1 * LAUNCH_SECONDS / seconds)))
             seen = torch.empty((2, 6), dtype=torch.float64, pin_memory=True)  # work[2:8] after the last two launches
             done = [torch.cuda.Event(), torch.cuda.Event()]
             launched, i = 0, 0
