@@ -344,7 +344,7 @@ class NISTGPU:
         return torch.from_numpy(np.asarray(x, np.float64)).to(self.asm.device)
 
     def _solve_pcg(self, K, R, dir_idx):
-        """Preconditioned CG on the device (efe_pcg_start / efe_pcg_iterate), nodal block-Jacobi or
+        """Preconditioned CG on the device (efe_pcg_start / efe_pcg_solve), nodal block-Jacobi or
         Jacobi (pcgPreconditioner).  The reference's
         system has identity rows for the Dirichlet DOFs; moving the known values to the right-hand
         side gives the same solution from the symmetric positive-definite system on the free DOFs:

@@ -77,7 +77,8 @@ enum {
                      element residual are formed in float-float arithmetic (~48-bit significand,
                      needs geomG32 and geomGlo); the Kirchhoff stress, state and the global
                      residual accumulation stay FP64 (small-strain solids and Hexa20 3x3x3 form
-                     their kinematics and residual in exact integer sums in every mode)         */
+                     their kinematics and residual in integer sums in every mode and do not read
+                     geomG32 and geomGlo, which this mode demands of all groups alike)          */
 };
 /* status words (int32[3], zeroed by the caller): status[0] = OR of EFE_STATUS_* bits,
    status[1] = INT32_MAX - (global index of the first failing element), 0 if none,
@@ -260,10 +261,12 @@ int32_t efe_compute_elements_persistent_noalloc(const EfeWorkItem* items, int32_
    (free_i = 1) and the identity on prescribed rows; K is read as assembled (double or float per
    kPrecision, int32 CSR), products accumulate in FP64.  efe_pcg_start sets x = 0, r = b,
    z = dinv r, p = z for a right-hand side b that is zero on the prescribed DOFs;
-   efe_pcg_iterate runs nIterations CG steps (firstIteration = the number already run, whose
-   parity selects the scalar buffers); work[2] then holds r.r for the convergence test (one
-   small device-to-host read per batch of iterations).  All vectors are caller-owned [n] device
-   arrays; work is EFE_PCG_WORK_DOUBLES doubles of caller-owned device scratch. */
+   efe_pcg_iterate runs nIterations CG steps in one launch (firstIteration = the number already
+   run, whose parity selects the scalar buffers); work[2] then holds r.r for the convergence test
+   and work[5] a negative value if a wait inside the kernel gave up (an internal error: x is
+   invalid, although the call returned EFE_OK), so both are read after a batch of iterations;
+   efe_pcg_solve tests on the device.  All vectors are caller-owned [n] device arrays (z is used by
+   efe_pcg_start only); work is EFE_PCG_WORK_DOUBLES doubles of caller-owned device scratch. */
 #define EFE_PCG_WORK_DOUBLES 6152
 typedef struct EfePcg {
   int64_t n;
@@ -287,8 +290,9 @@ typedef struct EfePcg {
   int32_t blockSize;       /* 1, 2 or 3 DOFs per preconditioner block (n a multiple of it)     */
   int32_t patternBlock;    /* 2 or 3: rows come in aligned groups of that many that share one
                               column list (a node's DOF rows; efe_pattern_fill's pattern when
-                              every node's first DOF is a multiple of it): the float-float
-                              product reads each column index once per group; 0 or 1: none */
+                              every node's first DOF is a multiple of it): with blockCols,
+                              efe_pcg_solve reads one column per node block; 0 or 1: none
+                              (efe_pcg_iterate reads one column per entry in any case)       */
 } EfePcg;
 /* y_i = free_i ? (K x)_i : x_i */
 int32_t efe_csr_spmv(const EfePcg* solver, const double* x, double* y, void* stream);
