@@ -1041,7 +1041,7 @@ def run_adjoint(args):
                      "median_rel_err": float(np.median(errs)) if errs else None},
         "pcg_iteration_ms": solve_ms / max(sum(pcg_its), 1),
         "roofline": dict(roofline_hbm(adj_bytes, adjoint_ms),
-                         fp64_pipe_active_pct=ncu_value("adjoint_tl_c3d8tl_16cube", "fp64_pipe_active_pct")),
+                         fp64_pipe_active_pct=ncu_value("adjoint_tl_c3d8tl_32cube", "fp64_pipe_active_pct")),
         "cpu_baseline": cpu,
         "e2e": {"value": 1e3 / e2e_ms, "unit": "grad/s", "h2d_bytes_per_step": 2 * nDof * 8,
                 "d2h_bytes_per_step": (len(coords) * 3 + nEl * 2) * 8, "ms_per_step": e2e_ms},

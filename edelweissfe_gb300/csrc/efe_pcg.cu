@@ -24,9 +24,13 @@
 // Precision: FP32 tangents multiply in float-float arithmetic against p held as float pairs (~48 bits, ff_madd),
 // FP64 tangents in FP64; vectors and scalars are FP64.
 //
-// Measured (one iteration, before: a product, an update and a direction kernel per iteration, replayed as a graph):
-// 64^3 Hexa8, FP32 values 212 -> 75 us (phase A 55 us for 288 MB, 5.2 TB/s; the two synchronisations 8, B 10),
-// 32^3 Hexa8, FP64 values 56.6 -> 29 us (phase A 16 us, its FP64 work alone 15); 40 x 8 plate 15.4 -> 7.0 us.
+// Measured (a solve's time by its iterations, set-up included; before: a product, an update and a direction kernel per
+// iteration, replayed as a graph): 64^3 Hexa8, FP32 values 208 -> 75 us (phase A 55 us for 288 MB, 5.2 TB/s; the two
+// synchronisations 8, B 10), 32^3 Hexa8, FP64 values 56 -> 31 us (phase A 16 us, its FP64 work alone 15); 40 x 8 plate 16.0
+// -> 6.0 us; Hexa20, whose corner nodes' chunks are longer than a copy, 24 x 24 x 12, FP32 48 -> 43 us, FP64 76 -> 53.
+//
+// The grid's scalars lie in slots of their epoch (efe_pcg_slots.cuh).  Every wait is bounded; one that gives up (about two
+// seconds) ends the launch with work[5] = -1.
 #include "efe_launch.cuh"
 #include "efe_pcg_slots.cuh"
 
